@@ -266,7 +266,8 @@ typedef struct rmn_batch_options {
   int32_t use_graph;     /* replay the wavefront iterations from captured CUDA graphs */
   int32_t pool_workers;  /* paths in flight per lane (0: library default, 2^22, halved while the workers
                             would take over a quarter of the free device memory) */
-  int32_t lanes;         /* independent wavefronts run side by side, 1..4 (0: library default, 3) */
+  int32_t lanes;         /* independent wavefronts run side by side, 1..4 (0: library default, one per 2^21 work
+                            units, 1 to 3). A batch of few units is rendered without them */
   int32_t stack_entries; /* traversal stack, 23 or 27 entries (0: library default, the smallest that holds
                             every item's tree: 23 when all trees are at most 22 levels deep); a stack too
                             small for a tree is RMN_ERR_INVALID_ARGUMENT */

@@ -26,6 +26,8 @@
 //                        of the ray queues with per-lane dynamic ray fetch.
 //     Traversal thus runs at the occupancy of a 64-register kernel, and the
 //     shading code runs on warps of one phase each.
+//     block_kernel    -- the end of a render, or a whole small one: the same
+//                        steps inside thread blocks, without launches.
 //  3. finalize_kernel -- per pixel, merges its units' partial accumulators
 //     in unit order and writes the four RadianceData buffers.
 //
@@ -148,7 +150,8 @@ __device__ __forceinline__ void store_diff(const Pool& P, int w, const RayDiff& 
 //   [6] (its Clum or -1, S, n, its sample id = slot * 8 + index in the path's samples)
 #define RMN_PART_F4 7
 
-enum Phase { PH_FETCH = 0, PH_SLOT, PH_WAIT_DIRECT, PH_WAIT_CLOSEST, PH_NEE, PH_WAIT_NEE, PH_DONE, PH_BOUNCE };
+enum Phase { PH_FETCH = 0, PH_SLOT, PH_WAIT_DIRECT, PH_WAIT_CLOSEST, PH_NEE, PH_WAIT_NEE, PH_DONE, PH_BOUNCE,
+             PH_LIGHT, PH_PATH };  // the last two only name slot_step's answer
 
 // First-vertex light samples a worker draws at once: consecutive direct
 // slots of its unit, each with its own shadow ray in the same queue.
@@ -370,14 +373,16 @@ __device__ __forceinline__ void push(int* q, unsigned int* qn, int w) { q[agg_in
 // Ray queues are double-buffered by iteration parity: the queues filled in
 // iteration i are traced in iteration i and consumed in iteration i + 1.
 
-// The light samples of a terminating vertex, drawn in order from the
-// path's stream: each that needs a shadow ray gets one of the worker's ray
-// slots (its sample index kept beside it). Returns the number queued.
-__device__ __forceinline__ int nee_draw(const Job* J, const Pool& P, int w, RmnRng& rng, int cnt) {
+// The light samples [k0, k1) of a terminating vertex (of its cnt), drawn in
+// order from the path's stream: each that needs a shadow ray gets one of the
+// worker's ray slots (its sample index kept beside it). n: the rays already
+// queued; returns them with the new ones.
+__device__ __forceinline__ int nee_draw(const Job* J, const Pool& P, int w, RmnRng& rng, const int4 nk, int k0,
+                                        int k1, int n) {
   const DevScene& s = J->s;
+  const int cnt = nk.y;
   const float4* nv = P.nv + 6 * (size_t)w;
   float4 a = nv[0], b = nv[1], c = nv[2], d = nv[3], e = nv[4], f = nv[5];
-  const int4 nk = P.nk[w];
   Surf sf = default_surf();
   sf.pos = f3(a.x, a.y, a.z);
   sf.shapeN = f3(b.x, b.y, b.z);
@@ -390,8 +395,7 @@ __device__ __forceinline__ int nee_draw(const Job* J, const Pool& P, int w, RmnR
   sf.entering = nk.z != 0;
   float4 l0 = P.lw[2 * w], l1 = P.lw[2 * w + 1];
   float lwt[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-  int n = 0;
-  for (int k = 0; k < cnt; ++k) {
+  for (int k = k0; k < k1; ++k) {
     float3 dir;
     float aim;
     LSample ls;
@@ -433,6 +437,7 @@ __device__ __forceinline__ void load_worker(const Pool& P, int w, int4& ph, int4
   uid = (long long)(((unsigned long long)(unsigned)b.w << 32) | (unsigned)b.z);
 }
 __device__ __forceinline__ int worker_job(const Pool& P, int w) { return P.hdr[2 * (size_t)w].x; }
+__device__ __forceinline__ int worker_phase(const Pool& P, int w) { return P.hdr[2 * (size_t)w + 1].y & 15; }
 __device__ __forceinline__ void store_worker(const Pool& P, int w, const int4& ph, int phase, const RmnRng& rng,
                                              const int4& un, long long uid) {
   P.hdr[2 * (size_t)w] = un;
@@ -582,6 +587,45 @@ __device__ __noinline__ int shade_hit_glass(const Job* J, const Pool& P, int w, 
   return shade_hit<true>(J, P, w, rng, ph, un, part, res, o, dir, status);
 }
 
+// The steps below advance one worker by one phase: the logic kernels run them
+// over their queues, block_kernel over those of its block. Each
+// leaves the worker's record in the pool and returns its next phase.
+//
+// sampleRay's body at the answer of the worker's closest-hit ray,
+// src/render.cpp:121-312.
+RMN_D int shade_step(const Job* __restrict__ jobs, const Pool& P, int w, float4* __restrict__ parts, int* status) {
+  int4 ph, un;
+  long long uid;
+  load_worker(P, w, ph, un, uid);
+  const Job* J = &jobs[un.x];
+  const Params& p = J->p;
+  const DevScene& s = J->s;
+  RmnRng rng;
+  rng.key = rmn_stream_key(p.seed, (uint32_t)un.y, (uint32_t)un.z);
+  rng.ctr = (unsigned)ph.y;
+  float4* part = parts + (size_t)uid * RMN_PART_F4;
+  float2 res = P.res[w];
+  int h = __float_as_int(res.x);
+  float4 o4 = P.ro[w], d4 = P.rd[w];
+  float3 o = f3(o4.x, o4.y, o4.z), dir = f3(d4.x, d4.y, d4.z);
+  const bool exclude = (ph.w & FL_EXCLUDE) != 0;
+  int phase = PH_SLOT;  // unless set below, the slot ends here
+  if (h == -2) {
+    atomicExch(status, 1);
+  } else if (h < 0) {
+    float4 pb = P.pb[w];
+    if (!exclude && s.sky_w)
+      emit(part, indirect_base_of(*J, un.y), P.pa[w], f3(pb.x, pb.y, pb.z), inv_spp_of(*J, un.y),
+           {f3(1.0f), sky_get(s, dir), 1.0f}, un.z * 8);
+  } else {
+    phase = p.glass ? shade_hit_glass(J, P, w, rng, ph, un, part, res, o, dir, status)
+                    : shade_hit<false>(J, P, w, rng, ph, un, part, res, o, dir, status);
+  }
+  if (phase == PH_SLOT) un.z++;
+  store_worker(P, w, ph, phase, rng, un, uid);
+  return phase;
+}
+
 __global__ void __launch_bounds__(128, 8) shade_kernel(const Job* __restrict__ jobs, Pool P, Queues Q, Ctl* ctl,
                                                        int par, float4* __restrict__ parts, int* status) {
   const unsigned n = ctl->q[par ^ 1].c;
@@ -589,36 +633,7 @@ __global__ void __launch_bounds__(128, 8) shade_kernel(const Job* __restrict__ j
   QLen* out = &ctl->q[par];
   for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
     const int w = in[idx];
-    int4 ph, un;
-    long long uid;
-    load_worker(P, w, ph, un, uid);
-    const Job* J = &jobs[un.x];
-    const Params& p = J->p;
-    const DevScene& s = J->s;
-    RmnRng rng;
-    rng.key = rmn_stream_key(p.seed, (uint32_t)un.y, (uint32_t)un.z);
-    rng.ctr = (unsigned)ph.y;
-    float4* part = parts + (size_t)uid * RMN_PART_F4;
-    // sampleRay's body, src/render.cpp:121-312
-    float2 res = P.res[w];
-    int h = __float_as_int(res.x);
-    float4 o4 = P.ro[w], d4 = P.rd[w];
-    float3 o = f3(o4.x, o4.y, o4.z), dir = f3(d4.x, d4.y, d4.z);
-    const bool exclude = (ph.w & FL_EXCLUDE) != 0;
-    int phase = PH_SLOT;  // unless set below, the slot ends here
-    if (h == -2) {
-      atomicExch(status, 1);
-    } else if (h < 0) {
-      float4 pb = P.pb[w];
-      if (!exclude && s.sky_w)
-        emit(part, indirect_base_of(*J, un.y), P.pa[w], f3(pb.x, pb.y, pb.z), inv_spp_of(*J, un.y),
-             {f3(1.0f), sky_get(s, dir), 1.0f}, un.z * 8);
-    } else {
-      phase = p.glass ? shade_hit_glass(J, P, w, rng, ph, un, part, res, o, dir, status)
-                      : shade_hit<false>(J, P, w, rng, ph, un, part, res, o, dir, status);
-    }
-    if (phase == PH_SLOT) un.z++;
-    store_worker(P, w, ph, phase, rng, un, uid);
+    const int phase = shade_step(jobs, P, w, parts, status);
     if (phase == PH_WAIT_CLOSEST) push(Q.c[par], &out->c, w);
     else if (phase == PH_NEE) push(Q.nee, &out->nee, w);
     else if (phase == PH_BOUNCE) push(Q.bounce, &out->bounce, w);
@@ -631,62 +646,111 @@ __global__ void __launch_bounds__(128, 8) shade_kernel(const Job* __restrict__ j
 // closest-hit ray, in the operations and order of shade_hit's own bounce
 // (pr = 1 and no absorption on an opaque surface). A warp here runs the
 // reflection sampler alone, not beside emission and light-sample starts.
+RMN_D int bounce_step(const Job* __restrict__ jobs, const Pool& P, int w) {
+  int4 ph, un;
+  long long uid;
+  load_worker(P, w, ph, un, uid);
+  const Params& p = jobs[un.x].p;
+  RmnRng rng;
+  rng.key = rmn_stream_key(p.seed, (uint32_t)un.y, (uint32_t)un.z);
+  rng.ctr = (unsigned)ph.y;
+  const float4* nv = P.nv + 6 * (size_t)w;
+  const float4 a = nv[0], b = nv[1], c = nv[2], d = nv[3], e = nv[4], f = nv[5];
+  Surf sf = default_surf();
+  sf.pos = f3(a.x, a.y, a.z);
+  sf.shapeN = f3(b.x, b.y, b.z);
+  sf.roughness = b.w;
+  sf.surfN = f3(c.x, c.y, c.z);
+  sf.metallic = c.w;
+  sf.base = f3(d.x, d.y, d.z);
+  sf.eta = d.w;
+  sf.specular = e.w;
+  sf.opacity = f.y;
+  const float3 V = f3(e.x, e.y, e.z);
+  const float p_rr = a.w, rf = f.x;
+  const bool nee = f.z != 0.0f;
+  const int depth = ph.z;
+  float3 nd, wv;
+  int nf = 0;
+  sample_reflect(sf, V, rng, nd, wv, nf);
+  wv = wv / 1.0f;  // / P_reflect (1 on an opaque surface)
+  if (nee) wv = wv / p_rr;
+  int phase = PH_SLOT;
+  if (any_finite3(nd) && depth != p.maxd) {
+    wv = wv * f3(1.0f);  // no absorption outside media
+    const float4 pb = P.pb[w];
+    float3 thr = f3(pb.x, pb.y, pb.z) * wv;
+    P.pb[w] = make_float4(thr.x, thr.y, thr.z, rf);
+    if (nf > 0) {
+      float4 pa = P.pa[w];
+      pa.w = pa.w * (1.0f / (float)(1 + nf));
+      P.pa[w] = pa;
+    }
+    P.ro[w] = make_float4(sf.pos.x, sf.pos.y, sf.pos.z, RMN_EPS);
+    P.rd[w] = make_float4(nd.x, nd.y, nd.z, INFINITY);
+    ph.z = depth + 1;
+    ph.w = nee ? FL_EXCLUDE : 0;
+    phase = PH_WAIT_CLOSEST;
+  }
+  if (phase == PH_SLOT) un.z++;
+  store_worker(P, w, ph, phase, rng, un, uid);
+  return phase;
+}
+
 __global__ void __launch_bounds__(128, 6) bounce_kernel(const Job* __restrict__ jobs, Pool P, Queues Q, Ctl* ctl,
                                                         int par) {
   QLen* out = &ctl->q[par];
   const unsigned n = out->bounce;
   for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
     const int w = Q.bounce[idx];
-    int4 ph, un;
-    long long uid;
-    load_worker(P, w, ph, un, uid);
-    const Params& p = jobs[un.x].p;
-    RmnRng rng;
-    rng.key = rmn_stream_key(p.seed, (uint32_t)un.y, (uint32_t)un.z);
-    rng.ctr = (unsigned)ph.y;
-    const float4* nv = P.nv + 6 * (size_t)w;
-    const float4 a = nv[0], b = nv[1], c = nv[2], d = nv[3], e = nv[4], f = nv[5];
-    Surf sf = default_surf();
-    sf.pos = f3(a.x, a.y, a.z);
-    sf.shapeN = f3(b.x, b.y, b.z);
-    sf.roughness = b.w;
-    sf.surfN = f3(c.x, c.y, c.z);
-    sf.metallic = c.w;
-    sf.base = f3(d.x, d.y, d.z);
-    sf.eta = d.w;
-    sf.specular = e.w;
-    sf.opacity = f.y;
-    const float3 V = f3(e.x, e.y, e.z);
-    const float p_rr = a.w, rf = f.x;
-    const bool nee = f.z != 0.0f;
-    const int depth = ph.z;
-    float3 nd, wv;
-    int nf = 0;
-    sample_reflect(sf, V, rng, nd, wv, nf);
-    wv = wv / 1.0f;  // / P_reflect (1 on an opaque surface)
-    if (nee) wv = wv / p_rr;
-    int phase = PH_SLOT;
-    if (any_finite3(nd) && depth != p.maxd) {
-      wv = wv * f3(1.0f);  // no absorption outside media
-      const float4 pb = P.pb[w];
-      float3 thr = f3(pb.x, pb.y, pb.z) * wv;
-      P.pb[w] = make_float4(thr.x, thr.y, thr.z, rf);
-      if (nf > 0) {
-        float4 pa = P.pa[w];
-        pa.w = pa.w * (1.0f / (float)(1 + nf));
-        P.pa[w] = pa;
-      }
-      P.ro[w] = make_float4(sf.pos.x, sf.pos.y, sf.pos.z, RMN_EPS);
-      P.rd[w] = make_float4(nd.x, nd.y, nd.z, INFINITY);
-      ph.z = depth + 1;
-      ph.w = nee ? FL_EXCLUDE : 0;
-      phase = PH_WAIT_CLOSEST;
-    }
-    if (phase == PH_SLOT) un.z++;
-    store_worker(P, w, ph, phase, rng, un, uid);
+    const int phase = bounce_step(jobs, P, w);
     if (phase == PH_WAIT_CLOSEST) push(Q.c[par], &out->c, w);
     else push(Q.slot, &out->slot, w);
   }
+}
+
+// A terminating vertex: draws its light samples. Returns the shadow rays it
+// queued (0: the slot has ended).
+RMN_D int nee_draw_step(const Job* __restrict__ jobs, const Pool& P, int w) {
+  int4 ph, un;
+  long long uid;
+  load_worker(P, w, ph, un, uid);
+  const Job* J = &jobs[un.x];
+  RmnRng rng;
+  rng.key = rmn_stream_key(J->p.seed, (uint32_t)un.y, (uint32_t)un.z);
+  rng.ctr = (unsigned)ph.y;
+  const int4 nk = P.nk[w];
+  const int queued = nee_draw(J, P, w, rng, nk, 0, nk.y, 0);
+  if (queued) P.dk[w] = make_int2(nk.y, queued);
+  else un.z++;
+  store_worker(P, w, ph, queued ? PH_WAIT_NEE : PH_SLOT, rng, un, uid);
+  return queued;
+}
+
+// The answered samples of a terminating vertex, emitted in sample order; the
+// slot has ended.
+RMN_D void nee_emit_step(const Job* __restrict__ jobs, const Pool& P, int w, float4* __restrict__ parts) {
+  int4 ph, un;
+  long long uid;
+  load_worker(P, w, ph, un, uid);
+  const Job* J = &jobs[un.x];
+  RmnRng rng;
+  rng.key = 0;
+  rng.ctr = (unsigned)ph.y;
+  const int2 dk = P.dk[w];
+  const float4 pa = P.pa[w], pb = P.pb[w];
+  const float3 base = indirect_base_of(*J, un.y);
+  const float inv_spp = inv_spp_of(*J, un.y);
+  float4* part = parts + (size_t)uid * RMN_PART_F4;
+  for (int k = 0; k < dk.y; ++k) {
+    const size_t rid = (size_t)w * kDirectBatch + k;
+    if (P.dres[rid] != 0.0f) continue;
+    float4 b0 = P.dpend[2 * rid], b1 = P.dpend[2 * rid + 1];
+    emit(part, base, pa, f3(pb.x, pb.y, pb.z), inv_spp, {f3(b0.x, b0.y, b0.z), f3(b1.x, b1.y, b1.z), b0.w},
+         un.z * 8 + __float_as_int(b1.w));
+  }
+  un.z++;
+  store_worker(P, w, ph, PH_SLOT, rng, un, uid);
 }
 
 __global__ void __launch_bounds__(128, 8) nee_kernel(const Job* __restrict__ jobs, Pool P, Queues Q, Ctl* ctl,
@@ -696,35 +760,9 @@ __global__ void __launch_bounds__(128, 8) nee_kernel(const Job* __restrict__ job
   const int* in = Q.nw[par ^ 1];
   for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
     const int w = idx < a ? in[idx] : Q.nee[idx - a];
-    int4 ph, un;
-    long long uid;
-    load_worker(P, w, ph, un, uid);
-    const Job* J = &jobs[un.x];
-    RmnRng rng;
-    rng.key = rmn_stream_key(J->p.seed, (uint32_t)un.y, (uint32_t)un.z);
-    rng.ctr = (unsigned)ph.y;
     int queued = 0;
-    if (ph.x == PH_WAIT_NEE) {
-      // the answered samples, emitted in sample order
-      const int2 dk = P.dk[w];
-      const float4 pa = P.pa[w], pb = P.pb[w];
-      const float3 base = indirect_base_of(*J, un.y);
-      const float inv_spp = inv_spp_of(*J, un.y);
-      float4* part = parts + (size_t)uid * RMN_PART_F4;
-      for (int k = 0; k < dk.y; ++k) {
-        const size_t rid = (size_t)w * kDirectBatch + k;
-        if (P.dres[rid] != 0.0f) continue;
-        float4 b0 = P.dpend[2 * rid], b1 = P.dpend[2 * rid + 1];
-        emit(part, base, pa, f3(pb.x, pb.y, pb.z), inv_spp, {f3(b0.x, b0.y, b0.z), f3(b1.x, b1.y, b1.z), b0.w},
-             un.z * 8 + __float_as_int(b1.w));
-      }
-    } else {
-      const int cnt = P.nk[w].y;
-      queued = nee_draw(J, P, w, rng, cnt);
-      if (queued) P.dk[w] = make_int2(cnt, queued);
-    }
-    if (!queued) un.z++;
-    store_worker(P, w, ph, queued ? PH_WAIT_NEE : PH_SLOT, rng, un, uid);
+    if (worker_phase(P, w) == PH_WAIT_NEE) nee_emit_step(jobs, P, w, parts);
+    else queued = nee_draw_step(jobs, P, w);
     if (queued) {
       push_rays(Q.sn[par], &out->sn, w, queued);
       push(Q.nw[par], &out->nw, w);
@@ -827,6 +865,82 @@ __device__ __forceinline__ void unit_of_fetch(const Params& p, long long local, 
 // vertex, leave the worker to the next iteration's slot_kernel. Results do
 // not depend on these hand-offs: every slot draws from its own stream and
 // adds into its own unit's record.
+//
+// Returns PH_LIGHT or PH_PATH, the kind of the worker's next slot, or PH_DONE.
+RMN_D int slot_step(const Job* __restrict__ jobs, int njobs, const Pool& P, int w, unsigned long long* next_unit,
+                    long long total_units, float4* __restrict__ parts) {
+  int4 ph, un;
+  long long uid;
+  load_worker(P, w, ph, un, uid);
+  int phase = ph.x;
+  const Job* J = phase == PH_FETCH ? nullptr : &jobs[un.x];
+  RmnRng rng;
+  rng.key = 0;
+  rng.ctr = (unsigned)ph.y;
+  if (phase == PH_WAIT_DIRECT) {
+    // the answered light samples of the batch, added in slot order
+    const int2 dk = P.dk[w];
+    const float3 base = base_of(*J, un.y);
+    float4* part = parts + (size_t)uid * RMN_PART_F4;
+    Rad4 dd = r4(part[0]), ds = r4(part[1]);
+    for (int k = 0; k < dk.y; ++k) {
+      const size_t rid = (size_t)w * kDirectBatch + k;
+      if (P.dres[rid] == 0.0f) {
+        float4 b0 = P.dpend[2 * rid], b1 = P.dpend[2 * rid + 1];
+        Rad4 d, sp;
+        demodulate(base, f3(b0.x, b0.y, b0.z), f3(b1.x, b1.y, b1.z), b0.w, d, sp);
+        radd(dd, d);
+        radd(ds, sp);
+      }
+    }
+    part[0] = f4(dd);
+    part[1] = f4(ds);
+    un.z += dk.x;
+    phase = PH_SLOT;
+  }
+  // fetch units until one has a slot left; every pass takes a new unit,
+  // so the loop ends within the units of the batch
+  for (;;) {
+    if (phase == PH_FETCH) {
+      unsigned long long u = agg_inc(next_unit);
+      if ((long long)u >= total_units) {
+        phase = PH_DONE;
+        break;
+      }
+      uid = (long long)u;
+      int jb = find_job_unit(jobs, njobs, uid);
+      J = &jobs[jb];
+      int pixel, sub;
+      unit_of_fetch(J->p, uid - J->unit_begin, pixel, sub);
+      uid = J->unit_begin + (long long)pixel * J->p.K + sub;  // the unit's record, in pixel order
+      const float* gb0 = gbuf_of(*J, pixel);
+      // 16 times the indirect samples behind a transmissive or half-opaque
+      // first vertex (renderPixel, src/render.cpp:497-499); the units of a
+      // scene with such materials are laid out for that many
+      const int pix_slots = (J->p.glass && !(gb0[17] > 1.0f - RMN_EPS)) ? J->p.slots16 : J->p.slots;
+      int j0, j1;
+      unit_slots(J->p, sub, pix_slots, j0, j1);
+      float4* part = parts + (size_t)uid * RMN_PART_F4;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) part[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      part[6] = make_float4(-1.0f, 0.0f, __int_as_float(0), __int_as_float(-1));
+      const float* gb = gbuf_of(*J, pixel);
+      bool hit = any_finite3(f3(gb[6], gb[7], gb[8]));
+      un = make_int4(jb, pixel, hit ? j0 : j1, j1);
+      phase = PH_SLOT;
+      continue;
+    }
+    if (un.z >= un.w) {
+      phase = PH_FETCH;
+      continue;
+    }
+    break;
+  }
+  store_worker(P, w, ph, phase, rng, un, uid);
+  if (phase == PH_DONE) return PH_DONE;
+  return un.z < J->p.spp_d ? PH_LIGHT : PH_PATH;
+}
+
 __global__ void __launch_bounds__(128, 8) slot_kernel(const Job* __restrict__ jobs, int njobs, Pool P, Queues Q,
                                                       Ctl* ctl, unsigned long long* next_unit, int par,
                                                       long long total_units, float4* __restrict__ parts) {
@@ -835,76 +949,9 @@ __global__ void __launch_bounds__(128, 8) slot_kernel(const Job* __restrict__ jo
   const int* in = Q.sd[par ^ 1];
   for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
     const int w = idx < a ? in[idx] : Q.slot[idx - a];
-    int4 ph, un;
-    long long uid;
-    load_worker(P, w, ph, un, uid);
-    int phase = ph.x;
-    const Job* J = phase == PH_FETCH ? nullptr : &jobs[un.x];
-    RmnRng rng;
-    rng.key = 0;
-    rng.ctr = (unsigned)ph.y;
-    if (phase == PH_WAIT_DIRECT) {
-      // the answered light samples of the batch, added in slot order
-      const int2 dk = P.dk[w];
-      const float3 base = base_of(*J, un.y);
-      float4* part = parts + (size_t)uid * RMN_PART_F4;
-      Rad4 dd = r4(part[0]), ds = r4(part[1]);
-      for (int k = 0; k < dk.y; ++k) {
-        const size_t rid = (size_t)w * kDirectBatch + k;
-        if (P.dres[rid] == 0.0f) {
-          float4 b0 = P.dpend[2 * rid], b1 = P.dpend[2 * rid + 1];
-          Rad4 d, sp;
-          demodulate(base, f3(b0.x, b0.y, b0.z), f3(b1.x, b1.y, b1.z), b0.w, d, sp);
-          radd(dd, d);
-          radd(ds, sp);
-        }
-      }
-      part[0] = f4(dd);
-      part[1] = f4(ds);
-      un.z += dk.x;
-      phase = PH_SLOT;
-    }
-    // fetch units until one has a slot left; every pass takes a new unit,
-    // so the loop ends within the units of the batch
-    for (;;) {
-      if (phase == PH_FETCH) {
-        unsigned long long u = agg_inc(next_unit);
-        if ((long long)u >= total_units) {
-          phase = PH_DONE;
-          break;
-        }
-        uid = (long long)u;
-        int jb = find_job_unit(jobs, njobs, uid);
-        J = &jobs[jb];
-        int pixel, sub;
-        unit_of_fetch(J->p, uid - J->unit_begin, pixel, sub);
-        uid = J->unit_begin + (long long)pixel * J->p.K + sub;  // the unit's record, in pixel order
-        const float* gb0 = gbuf_of(*J, pixel);
-        // 16 times the indirect samples behind a transmissive or half-opaque
-        // first vertex (renderPixel, src/render.cpp:497-499); the units of a
-        // scene with such materials are laid out for that many
-        const int pix_slots = (J->p.glass && !(gb0[17] > 1.0f - RMN_EPS)) ? J->p.slots16 : J->p.slots;
-        int j0, j1;
-        unit_slots(J->p, sub, pix_slots, j0, j1);
-        float4* part = parts + (size_t)uid * RMN_PART_F4;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) part[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        part[6] = make_float4(-1.0f, 0.0f, __int_as_float(0), __int_as_float(-1));
-        const float* gb = gbuf_of(*J, pixel);
-        bool hit = any_finite3(f3(gb[6], gb[7], gb[8]));
-        un = make_int4(jb, pixel, hit ? j0 : j1, j1);
-        phase = PH_SLOT;
-        continue;
-      }
-      if (un.z >= un.w) {
-        phase = PH_FETCH;
-        continue;
-      }
-      break;
-    }
-    store_worker(P, w, ph, phase, rng, un, uid);
+    const int phase = slot_step(jobs, njobs, P, w, next_unit, total_units, parts);
     if (phase == PH_DONE) continue;
-    if (un.z < J->p.spp_d) push(Q.light, &out->light, w);
+    if (phase == PH_LIGHT) push(Q.light, &out->light, w);
     else push(Q.path, &out->path, w);
   }
 }
@@ -912,6 +959,51 @@ __global__ void __launch_bounds__(128, 8) slot_kernel(const Job* __restrict__ jo
 // sampleDirectLightFromFirstIntersection, src/render.cpp:425-437: up to
 // kDirectBatch consecutive light-sample slots of the worker's unit at once,
 // each from its own stream; the samples without a shadow ray add nothing.
+// Returns the shadow rays queued (0: the worker is back in PH_SLOT).
+template <bool COUNT>
+RMN_D int light_step(const Job* __restrict__ jobs, const Pool& P, int w, unsigned long long& slots) {
+  int4 ph, un;
+  long long uid;
+  load_worker(P, w, ph, un, uid);
+  const Job* J = &jobs[un.x];
+  const Params& p = J->p;
+  const DevScene& s = J->s;
+  RmnRng rng;
+  rng.key = 0;
+  rng.ctr = (unsigned)ph.y;
+  Surf g = load_first_vertex(*J, un.y);
+  const int c = min(min(un.w, p.spp_d) - un.z, kDirectBatch);
+  if (COUNT) slots += (unsigned long long)c;
+  float3 Vd = -norm3(g.pos - p.pos);
+  float lwt[8];
+  float tot = 0.0f;
+  int nr = 0;
+  if (!(len3(g.emis) > 0.0f) && (s.sky_w != 0 || light_weights(s, g, Vd, lwt, tot))) {
+    for (int k = 0; k < c; ++k) {
+      RmnRng rk = rmn_rng(p.seed, (uint32_t)un.y, (uint32_t)(un.z + k));
+      float3 dir;
+      float aim;
+      LSample ls;
+      if (!light_gen(s, g, Vd, lwt, tot, p.spp_d, rk, dir, aim, ls)) continue;
+      const size_t rid = (size_t)w * kDirectBatch + nr++;
+      P.drd[rid] = make_float4(dir.x, dir.y, dir.z, aim);
+      P.dpend[2 * rid] = make_float4(ls.bsdf.x, ls.bsdf.y, ls.bsdf.z, ls.weight);
+      P.dpend[2 * rid + 1] = make_float4(ls.light.x, ls.light.y, ls.light.z, 0.0f);
+    }
+  }
+  int phase;
+  if (nr == 0) {
+    un.z += c;  // nothing to wait for: the next iteration's slot_kernel goes on
+    phase = PH_SLOT;
+  } else {
+    P.ro[w] = make_float4(g.pos.x, g.pos.y, g.pos.z, RMN_EPS);
+    P.dk[w] = make_int2(c, nr);
+    phase = PH_WAIT_DIRECT;
+  }
+  store_worker(P, w, ph, phase, rng, un, uid);
+  return nr;
+}
+
 template <bool COUNT>
 __global__ void __launch_bounds__(128, 8) light_kernel(const Job* __restrict__ jobs, Pool P, Queues Q, Ctl* ctl,
                                                        int par, Counters* ctr) {
@@ -920,46 +1012,8 @@ __global__ void __launch_bounds__(128, 8) light_kernel(const Job* __restrict__ j
   unsigned long long slots_done = 0;
   for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
     const int w = Q.light[idx];
-    int4 ph, un;
-    long long uid;
-    load_worker(P, w, ph, un, uid);
-    const Job* J = &jobs[un.x];
-    const Params& p = J->p;
-    const DevScene& s = J->s;
-    RmnRng rng;
-    rng.key = 0;
-    rng.ctr = (unsigned)ph.y;
-    Surf g = load_first_vertex(*J, un.y);
-    const int c = min(min(un.w, p.spp_d) - un.z, kDirectBatch);
-    if (COUNT) slots_done += (unsigned long long)c;
-    float3 Vd = -norm3(g.pos - p.pos);
-    float lwt[8];
-    float tot = 0.0f;
-    int nr = 0;
-    if (!(len3(g.emis) > 0.0f) && (s.sky_w != 0 || light_weights(s, g, Vd, lwt, tot))) {
-      for (int k = 0; k < c; ++k) {
-        RmnRng rk = rmn_rng(p.seed, (uint32_t)un.y, (uint32_t)(un.z + k));
-        float3 dir;
-        float aim;
-        LSample ls;
-        if (!light_gen(s, g, Vd, lwt, tot, p.spp_d, rk, dir, aim, ls)) continue;
-        const size_t rid = (size_t)w * kDirectBatch + nr++;
-        P.drd[rid] = make_float4(dir.x, dir.y, dir.z, aim);
-        P.dpend[2 * rid] = make_float4(ls.bsdf.x, ls.bsdf.y, ls.bsdf.z, ls.weight);
-        P.dpend[2 * rid + 1] = make_float4(ls.light.x, ls.light.y, ls.light.z, 0.0f);
-      }
-    }
-    int phase;
-    if (nr == 0) {
-      un.z += c;  // nothing to wait for: the next iteration's slot_kernel goes on
-      phase = PH_SLOT;
-    } else {
-      P.ro[w] = make_float4(g.pos.x, g.pos.y, g.pos.z, RMN_EPS);
-      P.dk[w] = make_int2(c, nr);
-      push_rays(Q.sn[par], &out->sn, w, nr);
-      phase = PH_WAIT_DIRECT;
-    }
-    store_worker(P, w, ph, phase, rng, un, uid);
+    const int nr = light_step<COUNT>(jobs, P, w, slots_done);
+    if (nr > 0) push_rays(Q.sn[par], &out->sn, w, nr);
     push(Q.sd[par], &out->sd, w);
   }
   if (COUNT && slots_done) atomicAdd(&ctr->slots, slots_done);
@@ -967,6 +1021,51 @@ __global__ void __launch_bounds__(128, 8) light_kernel(const Job* __restrict__ j
 
 // sampleIndirectLightFromFirstIntersection, src/render.cpp:314-423: the
 // first bounce of the unit's next path slot that has one.
+// Returns PH_WAIT_CLOSEST with the ray queued, or PH_SLOT when the unit's
+// remaining slots all end at the first vertex.
+template <bool COUNT>
+RMN_D int path_step(const Job* __restrict__ jobs, const Pool& P, int w, unsigned long long& slots) {
+  int4 ph, un;
+  long long uid;
+  load_worker(P, w, ph, un, uid);
+  const Job* J = &jobs[un.x];
+  const Params& p = J->p;
+  const DevScene& s = J->s;
+  RmnRng rng;
+  rng.key = 0;
+  rng.ctr = (unsigned)ph.y;
+  int phase = PH_SLOT;
+  while (un.z < un.w) {
+    Surf g = load_first_vertex(*J, un.y);
+    rng = rmn_rng(p.seed, (uint32_t)un.y, (uint32_t)un.z);
+    if (COUNT) slots++;
+    if (len3(g.emis) > 0.0f) {
+      un.z++;
+      continue;
+    }
+    float3 dir, w0;
+    int f0 = 0;
+    RayDiff d0;
+    if (s.has_tex) d0 = init_ray_diff(p, pixel_dir(p, un.y % p.W, un.y / p.W));
+    if (p.glass) first_bounce_glass(P, w, g, p.pos, rng, dir, w0, f0, s.has_tex ? &d0 : nullptr);
+    else first_bounce<false>(P, w, g, p.pos, rng, dir, w0, f0, s.has_tex ? &d0 : nullptr);
+    if (!any_finite3(dir)) {
+      un.z++;
+      continue;
+    }
+    P.pa[w] = make_float4(w0.x, w0.y, w0.z, f0 > 0 ? 1.0f / (float)(1 + f0) : 1.0f);
+    P.pb[w] = make_float4(1.0f, 1.0f, 1.0f, g.roughness * 1.0f);
+    P.ro[w] = make_float4(g.pos.x, g.pos.y, g.pos.z, RMN_EPS);
+    P.rd[w] = make_float4(dir.x, dir.y, dir.z, INFINITY);
+    ph.z = 1;           // depth of the vertex this ray will hit
+    ph.w = FL_EXCLUDE;  // the first bounce excludes direct light
+    phase = PH_WAIT_CLOSEST;
+    break;
+  }
+  store_worker(P, w, ph, phase, rng, un, uid);
+  return phase;
+}
+
 // 6 blocks per SM: the reflection sampler's registers (fewer spills) are
 // worth more here than occupancy (measured against 8: +0.8 % on batch64).
 template <bool COUNT>
@@ -977,44 +1076,7 @@ __global__ void __launch_bounds__(128, 6) path_kernel(const Job* __restrict__ jo
   unsigned long long slots_done = 0;
   for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
     const int w = Q.path[idx];
-    int4 ph, un;
-    long long uid;
-    load_worker(P, w, ph, un, uid);
-    const Job* J = &jobs[un.x];
-    const Params& p = J->p;
-    const DevScene& s = J->s;
-    RmnRng rng;
-    rng.key = 0;
-    rng.ctr = (unsigned)ph.y;
-    int phase = PH_SLOT;
-    while (un.z < un.w) {
-      Surf g = load_first_vertex(*J, un.y);
-      rng = rmn_rng(p.seed, (uint32_t)un.y, (uint32_t)un.z);
-      if (COUNT) slots_done++;
-      if (len3(g.emis) > 0.0f) {
-        un.z++;
-        continue;
-      }
-      float3 dir, w0;
-      int f0 = 0;
-      RayDiff d0;
-      if (s.has_tex) d0 = init_ray_diff(p, pixel_dir(p, un.y % p.W, un.y / p.W));
-      if (p.glass) first_bounce_glass(P, w, g, p.pos, rng, dir, w0, f0, s.has_tex ? &d0 : nullptr);
-      else first_bounce<false>(P, w, g, p.pos, rng, dir, w0, f0, s.has_tex ? &d0 : nullptr);
-      if (!any_finite3(dir)) {
-        un.z++;
-        continue;
-      }
-      P.pa[w] = make_float4(w0.x, w0.y, w0.z, f0 > 0 ? 1.0f / (float)(1 + f0) : 1.0f);
-      P.pb[w] = make_float4(1.0f, 1.0f, 1.0f, g.roughness * 1.0f);
-      P.ro[w] = make_float4(g.pos.x, g.pos.y, g.pos.z, RMN_EPS);
-      P.rd[w] = make_float4(dir.x, dir.y, dir.z, INFINITY);
-      ph.z = 1;           // depth of the vertex this ray will hit
-      ph.w = FL_EXCLUDE;  // the first bounce excludes direct light
-      phase = PH_WAIT_CLOSEST;
-      break;
-    }
-    store_worker(P, w, ph, phase, rng, un, uid);
+    const int phase = path_step<COUNT>(jobs, P, w, slots_done);
     if (phase == PH_WAIT_CLOSEST) push(Q.c[par], &out->c, w);
     else push(Q.sd[par], &out->sd, w);  // unit used up: the next iteration's slot_kernel fetches
   }
@@ -1205,6 +1267,337 @@ __global__ void __launch_bounds__(128, RMN_OCC_BLOCKS) qocc_kernel(const Job* __
 }
 
 
+// ------------------------------------------------- the wavefront in a block
+// block_kernel runs workers to the end of the render inside thread blocks:
+// each block owns up to kLocalWorkers of one lane's workers, keeps their
+// phases in queues in shared memory and fetches units until none is left. A
+// step of the block hands out tasks of up to 32 queue entries to its warps --
+// closest-hit rays with the shading of their answers, bounces, light samples
+// with their shadow rays, slot hand-offs, first bounces -- and every task
+// pushes what its workers do next into the queues of the following step. The
+// tasks run the logic kernels' own steps and traversals on the same records,
+// so the images are the wavefront's bit for bit.
+//
+// It takes the renders, and the ends of renders, that leave the wavefront
+// empty: an iteration of the wavefront costs 100-160 us however few workers
+// are left (nine launches in a row, each a chain of dependent loads 5-20 us
+// long), a step here 5-15 us, and a path needs about two steps a bounce.
+//
+// 256 threads and 256 workers a block, 80 registers (sample_reflect and
+// light_gen spill below that) and about 72 KB of shared memory: three blocks
+// per SM. The stacks and leaf exchanges of the two traversals share one
+// piece of shared memory per warp, which runs one of them at a time.
+constexpr int kLocalThreads = 256;
+constexpr int kLocalWorkers = 256;
+constexpr int kLocalBlocks = 3;  // per SM
+enum LocalQueue { LQ_RAY = 0, LQ_NEE, LQ_PATH, LQ_BOUNCE, LQ_SLOT, LQ_WAIT, LQ_WORKER_QUEUES };
+enum LocalItems { LI_LIGHT = 0, LI_SHADOW, LI_QUEUES };  // worker * kDirectBatch + sample
+constexpr int kLocalKinds = LQ_WORKER_QUEUES + LI_QUEUES;
+
+template <int STACK>
+union TravShared {  // of one warp
+  struct {
+    int2 stack[STACK * 32];
+    unsigned long long keys[32];
+  } closest;
+  struct {
+    int stack[STACK * 32];
+    OccExchangeT<32> x;
+  } occ;
+};
+
+template <int STACK>
+struct LocalShared {
+  TravShared<STACK> trav[kLocalThreads / 32];
+  uint16_t q[2][LQ_WORKER_QUEUES][kLocalWorkers];
+  uint16_t it[2][LI_QUEUES][kLocalWorkers * kDirectBatch];
+  int count[2][kLocalKinds];  // entries of q, then of it
+  int task;                   // next task of the step
+};
+
+// The lanes' closest-hit rays (all 32 lanes; `go`: the lane has worker w's):
+// the answers to the workers' records, as qtrace_kernel<false, ...>.
+template <bool ALPHA, int STACK>
+RMN_D void local_closest(const Job* __restrict__ jobs, const Pool& P, int w, bool go, TravShared<STACK>& sh,
+                         int* status) {
+  TRay r;
+  float tmin = 0.0f;
+  int searches = 0, jb = 0;
+  bool alpha = false, active = go;
+  const DevNode* nodes = nullptr;
+  const float4* tri = nullptr;
+  TravT<SharedStackN<STACK, 32>> t;
+  t.stack.base = sh.closest.stack + (threadIdx.x & 31);
+  t.ti = t.te = 0;
+  if (go) {
+    const float4 o = P.ro[w], d = P.rd[w];
+    jb = worker_job(P, w);
+    const DevScene& js = jobs[jb].s;
+    nodes = js.nodes;
+    tri = js.tri;
+    alpha = ALPHA && js.has_alpha != 0;
+    r = make_tray(f3(o.x, o.y, o.z), f3(d.x, d.y, d.z));
+    tmin = o.w;
+    trav_begin(js.root, t, d.w);
+  }
+  while (__ballot_sync(0xffffffffu, active) != 0) {
+    int st = coop_nodes<false>(nodes, r, tmin, t, active, kCoopSteps, nullptr);
+    if (coop_leaves<false, false>(tri, r, tmin, 0.0f, t, !alpha, sh.closest.keys)) st = 1;
+    if (!active || st == 0) continue;
+    if (ALPHA && st == 1 && alpha && alpha_again(jobs[jb].s, r, t, tmin, INFINITY, searches, true)) continue;
+    P.res[w] = make_float2(__int_as_float(st == -2 ? -2 : t.hit), t.tmax);
+    if (st == -2) atomicExch(status, 1);
+    active = false;
+  }
+}
+
+// The lanes' shadow rays (all 32 lanes; `go`: the lane has ray rid of worker
+// w), as qtrace_kernel<true, ...> or qocc_kernel.
+template <bool ALPHA, int STACK>
+RMN_D void local_shadow(const Job* __restrict__ jobs, const Pool& P, int w, size_t rid, bool go,
+                        TravShared<STACK>& sh, int* status) {
+  TRay r;
+  float tmin = 0.0f, aim = 0.0f;
+  int searches = 0, jb = 0, root = 0;
+  bool alpha = false, active = go;
+  const DevNode* nodes = nullptr;
+  const float4* tri = nullptr;
+  if (go) {
+    const float4 o = P.ro[w], d = P.drd[rid];
+    jb = worker_job(P, w);
+    const DevScene& js = jobs[jb].s;
+    nodes = js.nodes;
+    tri = js.tri;
+    root = js.root;
+    alpha = ALPHA && js.has_alpha != 0;
+    r = make_tray(f3(o.x, o.y, o.z), f3(d.x, d.y, d.z));
+    tmin = o.w;
+    aim = d.w;
+  }
+  if constexpr (ALPHA) {
+    TravT<SharedStackN<STACK, 32>> t;
+    t.stack.base = sh.closest.stack + (threadIdx.x & 31);
+    trav_begin(root, t, aim + RMN_EPS);
+    while (__ballot_sync(0xffffffffu, active) != 0) {
+      int st = coop_nodes<false>(nodes, r, tmin, t, active, kCoopSteps, nullptr);
+      if (coop_leaves<true, false>(tri, r, tmin, aim, t, !alpha, sh.closest.keys)) st = 1;
+      if (!active || st == 0) continue;
+      if (st == 1 && alpha && !(t.tmax >= aim) &&
+          alpha_again(jobs[jb].s, r, t, tmin, aim + RMN_EPS, searches, false))
+        continue;
+      P.dres[rid] = (st == -2 || t.tmax >= aim) ? 0.0f : 1.0f;
+      if (st == -2) atomicExch(status, 1);
+      active = false;
+    }
+  } else {
+    OccT<SharedStackRefN<STACK, 32>> t;
+    t.stack.base = sh.occ.stack + (threadIdx.x & 31);
+    occ_begin(root, t);
+    while (__ballot_sync(0xffffffffu, active) != 0) {
+      const int st = occ_nodes<false>(nodes, r, tmin, aim + RMN_EPS, t, active, kOccSteps, nullptr);
+      const bool occ = occ_leaves<false>(tri, r, tmin, aim, t, sh.occ.x);
+      if (!active || (st == 0 && !occ)) continue;
+      P.dres[rid] = (occ && st != -2) ? 1.0f : 0.0f;
+      if (st == -2) atomicExch(status, 1);
+      active = false;
+    }
+  }
+}
+
+// Sample k of the batch of first-vertex light samples that slot_step found
+// next for worker w: light_step's, one sample a lane. Returns whether it has
+// a shadow ray; a sample without one is put down as occluded and adds
+// nothing.
+RMN_D bool light_item(const Job* __restrict__ jobs, const Pool& P, int w, int k) {
+  int4 ph, un;
+  long long uid;
+  load_worker(P, w, ph, un, uid);
+  const Job* J = &jobs[un.x];
+  const Params& p = J->p;
+  const DevScene& s = J->s;
+  Surf g = load_first_vertex(*J, un.y);
+  float3 Vd = -norm3(g.pos - p.pos);
+  float lwt[8];
+  float tot = 0.0f;
+  const size_t rid = (size_t)w * kDirectBatch + k;
+  if (!(len3(g.emis) > 0.0f) && (s.sky_w != 0 || light_weights(s, g, Vd, lwt, tot))) {
+    RmnRng rk = rmn_rng(p.seed, (uint32_t)un.y, (uint32_t)(un.z + k));
+    float3 dir;
+    float aim;
+    LSample ls;
+    if (light_gen(s, g, Vd, lwt, tot, p.spp_d, rk, dir, aim, ls)) {
+      P.drd[rid] = make_float4(dir.x, dir.y, dir.z, aim);
+      P.dpend[2 * rid] = make_float4(ls.bsdf.x, ls.bsdf.y, ls.bsdf.z, ls.weight);
+      P.dpend[2 * rid + 1] = make_float4(ls.light.x, ls.light.y, ls.light.z, 0.0f);
+      return true;
+    }
+  }
+  P.dres[rid] = 1.0f;
+  return false;
+}
+
+// The batch itself: up to kDirectBatch light-sample slots of worker w's
+// unit. Returns their number.
+RMN_D int light_batch(const Job* __restrict__ jobs, const Pool& P, int w) {
+  int4 ph, un;
+  long long uid;
+  load_worker(P, w, ph, un, uid);
+  const Job& J = jobs[un.x];
+  const int c = min(min(un.w, J.p.spp_d) - un.z, kDirectBatch);
+  const float* gb = gbuf_of(J, un.y);
+  P.ro[w] = make_float4(gb[6], gb[7], gb[8], RMN_EPS);
+  P.dk[w] = make_int2(c, c);
+  RmnRng rng;
+  rng.key = 0;
+  rng.ctr = (unsigned)ph.y;
+  store_worker(P, w, ph, PH_WAIT_DIRECT, rng, un, uid);
+  return c;
+}
+
+// The next light sample of a terminating vertex, one a task: nee_draw_step
+// draws them all at once, four times as long as any other task. Returns the
+// ray slot of its shadow ray or -1; `more`: samples are left.
+RMN_D int nee_item(const Job* __restrict__ jobs, const Pool& P, int w, bool& more) {
+  int4 ph, un;
+  long long uid;
+  load_worker(P, w, ph, un, uid);
+  const Job* J = &jobs[un.x];
+  RmnRng rng;
+  rng.key = rmn_stream_key(J->p.seed, (uint32_t)un.y, (uint32_t)un.z);
+  rng.ctr = (unsigned)ph.y;
+  int4 nk = P.nk[w];
+  const int k = nk.x, had = k > 0 ? P.dk[w].y : 0;
+  const int n = nee_draw(J, P, w, rng, nk, k, k + 1, had);
+  more = k + 1 < nk.y;
+  nk.x = k + 1;
+  P.nk[w] = nk;
+  P.dk[w] = make_int2(nk.y, n);
+  if (!more && n == 0) un.z++;
+  store_worker(P, w, ph, more ? PH_NEE : n > 0 ? PH_WAIT_NEE : PH_SLOT, rng, un, uid);
+  return n > had ? had : -1;
+}
+
+template <bool ALPHA, int STACK>
+__global__ void __launch_bounds__(kLocalThreads, kLocalBlocks)
+    block_kernel(const Job* __restrict__ jobs, int njobs, Pool P, Queues Q, const Ctl* __restrict__ ctl,
+                 int per_block, unsigned long long* next_unit, long long total_units, float4* __restrict__ parts,
+                 int* status) {
+  extern __shared__ __align__(16) unsigned char local_shared[];
+  LocalShared<STACK>& sh = *reinterpret_cast<LocalShared<STACK>*>(local_shared);
+  TravShared<STACK>& trav = sh.trav[threadIdx.x >> 5];
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  // the workers waiting at the end of an iteration of parity 1, their rays
+  // answered: worker[k] is the one behind the queues' entry k
+  __shared__ int worker[kLocalWorkers];
+  const unsigned nc = ctl->q[1].c, nd = ctl->q[1].sd, nn = ctl->q[1].nw;
+  const unsigned first = blockIdx.x * (unsigned)per_block;
+  if (threadIdx.x < 2 * kLocalKinds) (&sh.count[0][0])[threadIdx.x] = 0;
+  if (threadIdx.x == 0) sh.task = 0;
+  __syncthreads();
+  int cur = 0;
+  // one atomic per lane: the lanes of a task push into different queues
+  auto push_worker = [&](int buf, int kind, int k) {
+    sh.q[buf][kind][atomicAdd(&sh.count[buf][kind], 1)] = (uint16_t)k;
+  };
+  auto push_lights = [&](int buf, int k, int n) {
+    const int at = atomicAdd(&sh.count[buf][LQ_WORKER_QUEUES + LI_LIGHT], n);
+    for (int j = 0; j < n; ++j) sh.it[buf][LI_LIGHT][at + j] = (uint16_t)(k * kDirectBatch + j);
+  };
+  // what follows a shading step
+  auto after_shade = [&](int buf, int k, int ph) {
+    if (ph == PH_WAIT_CLOSEST) push_worker(buf, LQ_RAY, k);
+    else if (ph == PH_NEE) push_worker(buf, LQ_NEE, k);
+    else if (ph == PH_BOUNCE) push_worker(buf, LQ_BOUNCE, k);
+    else push_worker(buf, LQ_SLOT, k);
+  };
+  for (int k = threadIdx.x; k < per_block; k += kLocalThreads) {
+    const unsigned i = first + k;
+    if (i >= nc + nd + nn) break;
+    worker[k] = i < nc ? Q.c[1][i] : i - nc < nd ? Q.sd[1][i - nc] : Q.nw[1][i - nc - nd];
+    // an answered closest-hit ray is traced once more, to the same answer:
+    // its shading follows in that task
+    push_worker(cur, i < nc ? LQ_RAY : LQ_SLOT, k);
+  }
+  __syncthreads();
+  unsigned long long unused = 0;
+  for (;;) {
+    int* count = sh.count[cur];
+    const int nxt = cur ^ 1;
+    int total = 0;
+#pragma unroll
+    for (int kind = 0; kind < kLocalKinds; ++kind) total += (count[kind] + 31) >> 5;
+    if (total == 0) break;
+    for (;;) {
+      int task = 0;
+      if (lane == 0) task = atomicAdd(&sh.task, 1);
+      task = __shfl_sync(FULL, task, 0);
+      if (task >= total) break;
+      // the longest tasks first
+      int kind = LQ_RAY, at = task, n = count[LQ_RAY];
+      constexpr int order[kLocalKinds] = {LQ_RAY, LQ_WORKER_QUEUES + LI_LIGHT, LQ_NEE,
+                                          LQ_WORKER_QUEUES + LI_SHADOW, LQ_PATH, LQ_BOUNCE, LQ_SLOT, LQ_WAIT};
+#pragma unroll
+      for (int o = 0; o < kLocalKinds; ++o) {
+        kind = order[o];
+        n = count[kind];
+        const int tasks = (n + 31) >> 5;
+        if (at < tasks) break;
+        at -= tasks;
+      }
+      const int e = at * 32 + lane;
+      const bool go = e < n;
+      if (kind >= LQ_WORKER_QUEUES) {
+        const int item = go ? sh.it[cur][kind - LQ_WORKER_QUEUES][e] : 0;
+        const int k = item / kDirectBatch, j = item % kDirectBatch;
+        const int w = worker[k];
+        bool ray = go;
+        if (kind == LQ_WORKER_QUEUES + LI_LIGHT) {
+          ray = go && light_item(jobs, P, w, j);
+          // the worker's answers are there when this step ends
+          if (go && j == 0) push_worker(nxt, LQ_SLOT, k);
+        }
+        __syncwarp();
+        if (__any_sync(FULL, ray))
+          local_shadow<ALPHA, STACK>(jobs, P, w, (size_t)w * kDirectBatch + j, ray, trav, status);
+      } else {
+        const int k = go ? sh.q[cur][kind][e] : 0;
+        const int w = worker[k];
+        if (kind == LQ_RAY) {
+          local_closest<ALPHA, STACK>(jobs, P, w, go, trav, status);
+          if (go) after_shade(nxt, k, shade_step(jobs, P, w, parts, status));
+        } else if (!go) {
+        } else if (kind == LQ_BOUNCE) {
+          push_worker(nxt, bounce_step(jobs, P, w) == PH_WAIT_CLOSEST ? LQ_RAY : LQ_SLOT, k);
+        } else if (kind == LQ_PATH) {
+          push_worker(nxt, path_step<false>(jobs, P, w, unused) == PH_WAIT_CLOSEST ? LQ_RAY : LQ_SLOT, k);
+        } else if (kind == LQ_NEE) {
+          bool more;
+          const int j = nee_item(jobs, P, w, more);
+          if (j >= 0)
+            sh.it[nxt][LI_SHADOW][atomicAdd(&sh.count[nxt][LQ_WORKER_QUEUES + LI_SHADOW], 1)] =
+                (uint16_t)(k * kDirectBatch + j);
+          push_worker(nxt, more ? LQ_NEE : LQ_WAIT, k);
+        } else if (kind == LQ_SLOT) {
+          if (worker_phase(P, w) == PH_WAIT_NEE) nee_emit_step(jobs, P, w, parts);
+          const int ph = slot_step(jobs, njobs, P, w, next_unit, total_units, parts);
+          if (ph == PH_LIGHT) push_lights(nxt, k, light_batch(jobs, P, w));
+          else if (ph == PH_PATH) push_worker(nxt, LQ_PATH, k);
+        } else {  // LQ_WAIT: the worker's last shadow ray is traced in this step
+          push_worker(nxt, LQ_SLOT, k);
+        }
+      }
+      __syncwarp();
+    }
+    __syncthreads();  // the step's queues are read, its records written
+    if (threadIdx.x < kLocalKinds) sh.count[cur][threadIdx.x] = 0;
+    if (threadIdx.x == 0) sh.task = 0;
+    cur = nxt;
+    __syncthreads();
+  }
+}
+
+
 // Ray binning (batch option ray_order): before a traversal launch, its queue
 // is reordered by a bucket key -- the ray's job, the octant of its direction
 // and a cell of its origin in an 8 x 8 x 8 grid over the job's scene box --
@@ -1367,8 +1760,12 @@ int blocks_per_sm(K kernel) {
 namespace rmn {
 
 
-constexpr int kDefaultLanes = 3;
-constexpr int kIterationsPerChunk = 8;
+// Iterations between two looks at the live workers. The end of a render goes
+// to block_kernel at the first look that finds few enough, so looks are
+// frequent: 2 against 8 iterations, 256x256 Cornell, 16 spp: 2.35 against 2.6
+// ms; ten uneven renders in one batch 12.6 against 14.0; a look costs about
+// 20 us, a 1080p frame of 64 spp takes 61.8 ms with either.
+constexpr int kIterationsPerChunk = 2;
 constexpr long long kMaxIterations = 1LL << 22;  // bound on the iteration loop; a finite render never reaches it
 
 struct JobTable {
@@ -1389,6 +1786,7 @@ struct BatchState {
   bool alpha = false;         // some job's scene has alpha-tested materials
   bool tex = false;           // some job's scene has textures
   bool shallow = true;        // the traversal runs its RMN_STACK_SMALL-entry build
+  bool direct = false;        // few units: block_kernel renders them all, without wavefront iterations
   Pool pool[kMaxLanes] = {};  // each lane's share of the worker arrays
   Queues q[kMaxLanes] = {};
   // ray binning (ray_order): per lane, the reordered closest and shadow
@@ -1412,6 +1810,13 @@ struct BatchState {
   cudaEvent_t upd = nullptr;
 };
 
+
+// Lanes of a batch that leaves them open: one per 2^21 units, 1 to 3. Lanes
+// overlap one another's kernels where each fills the device (1080p terrain,
+// 33 M units: 61.5 ms with three against 64.7 with one); with fewer workers
+// they only split them into emptier launches (Cornell 256x256, 64 spp, 1.05 M
+// units: 4.6 ms against 4.4; 16 spp: 2.75 against 2.35).
+static int default_lanes(long long units) { return (int)std::min<long long>(3, std::max<long long>(1, units >> 21)); }
 
 // Jobs ordered by decreasing depth (the longest paths start first), so the
 // pool drains on cheap units; results do not depend on the order.
@@ -1540,6 +1945,57 @@ static cudaError_t launch_iteration(BatchState* b, int lane, cudaStream_t st, Co
   return cudaGetLastError();
 }
 
+// The workers that block_kernel holds on the device at once. A render of no
+// more units runs in it from the start, and a longer one ends in it once no
+// unit is left and no more workers live: below this line the wavefront's
+// kernels are mostly latency, above it block_kernel's blocks would queue up.
+// Measured (Cornell 160x90, 4 spp, 28,800 units: 0.87 ms against 2.1 ms with
+// two wavefront iterations first; 256x256, 16 spp, 328 k units: 3.8 against
+// 2.35; the glass box 250x250, 16 spp ended at 60-120 k workers: 9.3-9.7 ms, at
+// 250 k: 11.9).
+static long long block_capacity() { return (long long)device_sms() * kLocalBlocks * kLocalWorkers; }
+
+// block_kernel over the n workers of one lane that wait at the end of an
+// iteration of parity 1, or were seeded.
+static cudaError_t launch_block(BatchState* b, int lane, long long n, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  const int nj = (int)b->table.jobs.size();
+  const int sms = device_sms();
+  // one block per SM while its queues hold its share of the workers: fuller
+  // queues make fuller tasks
+  const int per_block = (int)std::min<long long>(kLocalWorkers, std::max<long long>(64, (n + sms - 1) / sms));
+  const unsigned grid = (unsigned)((n + per_block - 1) / per_block);
+  Ctl* ctl = &b->d_ctl->lane[lane];
+  cudaError_t e = cudaSuccess;
+  auto go = [&](auto kernel, size_t bytes) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return;
+    kernel<<<grid, kLocalThreads, bytes, st>>>(b->d_jobs, nj, b->pool[lane], b->q[lane], ctl, per_block,
+                                               &b->d_ctl->next_unit, b->table.total_units, b->d_parts, b->d_status);
+    e = cudaGetLastError();
+  };
+  constexpr size_t small = sizeof(LocalShared<RMN_STACK_SMALL>), large = sizeof(LocalShared<RMN_STACK>);
+  if (b->alpha && b->shallow) go(block_kernel<true, RMN_STACK_SMALL>, small);
+  else if (b->alpha) go(block_kernel<true, RMN_STACK>, large);
+  else if (b->shallow) go(block_kernel<false, RMN_STACK_SMALL>, small);
+  else go(block_kernel<false, RMN_STACK>, large);
+  return e;
+}
+
+// The last workers of every lane (n[l] of lane l), the lanes side by side.
+static cudaError_t launch_blocks(BatchState* b, const long long* n, cudaStream_t st) {
+  cudaError_t e = cudaEventRecord(b->fork, st);
+  for (int l = 0; l < b->lanes && e == cudaSuccess; ++l) {
+    if (n[l] <= 0) continue;
+    cudaStream_t ls = l == 0 ? st : b->ls[l];
+    if (l > 0) e = cudaStreamWaitEvent(ls, b->fork, 0);
+    if (e == cudaSuccess) e = launch_block(b, l, n[l], ls);
+    if (l > 0 && e == cudaSuccess) e = cudaEventRecord(b->join[l], ls);
+    if (l > 0 && e == cudaSuccess) e = cudaStreamWaitEvent(st, b->join[l], 0);
+  }
+  return e;
+}
+
 static cudaError_t launch_finalize(BatchState* b, cudaStream_t st) {
   const int nj = (int)b->table.jobs.size(), tp = b->table.total_pix;
   finalize_kernel<<<(tp + 127) / 128, 128, 0, st>>>(b->d_jobs, nj, tp, b->d_parts);
@@ -1559,9 +2015,6 @@ static cudaError_t capture(cudaStream_t cs, F&& body, cudaGraphExec_t* out) {
   return e;
 }
 
-// The whole render: init (counters, pool, G-buffer), iterations in chunks
-// until every worker has retired, finalize. The host reads the live-worker
-// count after each chunk; kMaxIterations bounds the loop.
 // One chunk of iterations of every lane. Without counters or per-kernel
 // events the lanes run side by side on their own streams (forked from and
 // joined back into st); otherwise one after the other on st.
@@ -1584,15 +2037,36 @@ static cudaError_t launch_lanes(BatchState* b, cudaStream_t st, Counters* ctr, c
   return e;
 }
 
+// A whole render of few units.
+static cudaError_t launch_direct(BatchState* b, cudaStream_t st) {
+  cudaError_t e = launch_init(b, st, nullptr);
+  for (int l = 0; l < b->lanes && e == cudaSuccess; ++l) e = launch_block(b, l, b->pool[l].W, st);
+  return e == cudaSuccess ? launch_finalize(b, st) : e;
+}
+
 struct KernelTimes {
   double logic_ms = 0.0, trace_ms = 0.0;
   long long iterations = 0;
   cudaEvent_t e[kIterationsPerChunk][kMaxLanes][4] = {};
 };
 
+// The whole render: init (counters, pool, G-buffer), iterations in chunks
+// until few enough workers are left for block_kernel (or, in a profile, none),
+// finalize. The host reads the live-worker count after each chunk;
+// kMaxIterations bounds the loop.
 static rmn_status run(BatchState* b, cudaStream_t st, Counters* ctr, cudaEvent_t* ev, KernelTimes* kt = nullptr) {
   const bool graph = b->use_graph && !ctr && !kt;
+  // the profile's runs count and time the wavefront alone
+  const bool drain = !ctr && !kt;  // block_kernel takes the end
   cudaError_t e;
+  if (b->direct && drain) {
+    if (graph) {
+      e = cudaGraphLaunch(b->init_exec, st);
+    } else {
+      e = launch_direct(b, st);
+    }
+    return e == cudaSuccess ? RMN_OK : cuda_fail(e, "render");
+  }
   if (ev) cudaEventRecord(ev[0], st);
   e = graph ? cudaGraphLaunch(b->init_exec, st) : launch_init(b, st, ctr);
   if (e != cudaSuccess) return cuda_fail(e, "render init");
@@ -1618,7 +2092,17 @@ static rmn_status run(BatchState* b, cudaStream_t st, Counters* ctr, cudaEvent_t
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "render iteration");
     live = 0;
-    for (int l = 0; l < b->lanes; ++l) live += h.lane[l].q[1].c + h.lane[l].q[1].sd + h.lane[l].q[1].nw;
+    long long waiting[kMaxLanes] = {};
+    for (int l = 0; l < b->lanes; ++l) {
+      waiting[l] = (long long)h.lane[l].q[1].c + h.lane[l].q[1].sd + h.lane[l].q[1].nw;
+      live += (unsigned)waiting[l];
+    }
+    if (drain && live > 0 && (long long)live <= block_capacity() &&
+        (long long)h.next_unit >= b->table.total_units) {
+      e = launch_blocks(b, waiting, st);
+      if (e != cudaSuccess) return cuda_fail(e, "render tail");
+      break;
+    }
     if (kt) {
       for (int k = 0; k < kIterationsPerChunk; ++k)
         for (int l = 0; l < b->lanes; ++l) {
@@ -1632,9 +2116,9 @@ static rmn_status run(BatchState* b, cudaStream_t st, Counters* ctr, cudaEvent_t
     }
     // Every iteration answers every queued ray, so a chunk that neither
     // retires a worker nor hands out a unit is only possible while paths are
-    // long; 4096 such chunks in a row (>32k bounces) means no progress.
+    // long; 32768 such iterations in a row (as many bounces) mean no progress.
     if (live == last_live && h.next_unit == last_next) {
-      if (++stalled > 4096) return fail(RMN_ERR_DEVICE_LIMIT, "render: no progress over 32768 iterations");
+      if ((stalled += kIterationsPerChunk) > 32768) return fail(RMN_ERR_DEVICE_LIMIT, "render: no progress over 32768 iterations");
     } else {
       stalled = 0;
     }
@@ -1748,7 +2232,7 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
   b->table.slots = S_def;
   b->use_graph = use_graph;
   b->binned = ray_order != 0;
-  b->lanes = lanes > 0 ? std::min(lanes, kMaxLanes) : kDefaultLanes;
+  b->lanes = lanes > 0 ? std::min(lanes, kMaxLanes) : default_lanes(b->table.total_units);
   // workers per lane; no more lanes and workers than there are units; the
   // default pool halves while the workers would take more than a quarter of
   // the free device memory
@@ -1762,6 +2246,8 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
     const size_t budget = free_device_bytes() / 4;
     while (per > 4096 && worker_bytes(glass, tex) * (size_t)per * b->lanes > budget) per /= 2;
   }
+  b->direct = b->table.total_units <= block_capacity();
+  if (b->direct) b->lanes = 1;
   while (b->lanes > 1 && (long long)b->lanes * 128 > b->table.total_units) --b->lanes;
   per = std::min<long long>(per, (b->table.total_units + b->lanes - 1) / b->lanes);
   if (per < 1) per = 1;
@@ -1863,7 +2349,7 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
     // One chunk graph: the lanes' iterations as parallel branches (fork and
     // join through events between the lane streams), so their kernels overlap.
     cudaStream_t c0 = b->ls[0];
-    e = capture(c0, [&] { return launch_init(b, c0, nullptr); }, &b->init_exec);
+    e = capture(c0, [&] { return b->direct ? launch_direct(b, c0) : launch_init(b, c0, nullptr); }, &b->init_exec);
     if (e == cudaSuccess) e = capture(c0, [&] { return launch_lanes(b, c0, nullptr, nullptr); }, &b->chunk_exec);
     if (e == cudaSuccess) e = capture(c0, [&] { return launch_finalize(b, c0); }, &b->fin_exec);
   }
@@ -1936,7 +2422,7 @@ size_t batch_device_bytes(const RenderItem* items_in, int n, int pool_workers, i
     glass = glass || j.p.glass;
     tex = tex || j.s.has_tex;
   }
-  const int nl = lanes > 0 ? std::min(lanes, kMaxLanes) : kDefaultLanes;
+  const int nl = lanes > 0 ? std::min(lanes, kMaxLanes) : default_lanes(t.total_units);
   long long per = pool_workers > 0 ? pool_workers : kDefaultPoolWorkers;
   per = std::min<long long>(per, (t.total_units + nl - 1) / nl);
   // binning: the reordered queues and each entry's bucket, per worker; the

@@ -123,29 +123,30 @@ struct TraceCounters {
 // traversing.
 // Stack storage: per-thread local memory, or a slice of shared memory (the
 // persistent traversal kernels; entry e of thread i at base[e * 128 + i], so
-// a warp's accesses to one level fall in distinct banks). kCap entries.
+// a warp's accesses to one level fall in distinct banks; 32 instead of 128
+// where every warp has a stack array of its own). kCap entries.
 struct LocalStack {
   static constexpr int kCap = RMN_STACK;
   int2 e[RMN_STACK];  // (reference, entry distance as float bits)
   RMN_D void put(int i, int2 v) { e[i] = v; }
   RMN_D int2 get(int i) const { return e[i]; }
 };
-template <int N = RMN_STACK>
+template <int N = RMN_STACK, int STRIDE = 128>
 struct SharedStackN {
   static constexpr int kCap = N;
   int2* base;
-  RMN_D void put(int i, int2 v) { base[i * 128] = v; }
-  RMN_D int2 get(int i) const { return base[i * 128]; }
+  RMN_D void put(int i, int2 v) { base[i * STRIDE] = v; }
+  RMN_D int2 get(int i) const { return base[i * STRIDE]; }
 };
 using SharedStack = SharedStackN<RMN_STACK>;
 // References only (order-free occlusion): get() reports an entry distance of
 // -inf, so a pop never skips an entry.
-template <int N>
+template <int N, int STRIDE = 128>
 struct SharedStackRefN {
   static constexpr int kCap = N;
   int* base;
-  RMN_D void put(int i, int2 v) { base[i * 128] = v.x; }
-  RMN_D int2 get(int i) const { return make_int2(base[i * 128], __float_as_int(-INFINITY)); }
+  RMN_D void put(int i, int2 v) { base[i * STRIDE] = v.x; }
+  RMN_D int2 get(int i) const { return make_int2(base[i * STRIDE], __float_as_int(-INFINITY)); }
 };
 
 template <class Stack>
@@ -533,30 +534,33 @@ RMN_D int occ_nodes(const DevNode* __restrict__ nodes, const TRay& r, float tmin
   return res;
 }
 
-// The leaf phase's exchange in shared memory, per 128-thread block: each
-// lane with pending triangles writes its ray, its leaves and (batch
+// The leaf phase's exchange in shared memory, per 128-thread block (or, with
+// THREADS = 32, per warp): each lane with pending triangles writes its ray, its leaves and (batch
 // kernels) its triangle array once, and its lane index into its warp's
 // owner table for each of its triangles; the lane testing triangle k of the
 // warp's list reads its owner and the owner's data from there.
 constexpr int kOccOwn = 32 * 30;  // per warp: 32 lanes x two leaves of at most 15 triangles
-struct OccExchange {
-  float4 ray[2 * 128];         // (origin, aim), (direction, t_min)
-  int4 leaf[128];              // a0, c0, a1, first index of the lane's triangles in the warp's list
-  const float4* tri[128];
-  unsigned char own[4][kOccOwn];
+template <int THREADS>
+struct OccExchangeT {
+  float4 ray[2 * THREADS];     // (origin, aim), (direction, t_min)
+  int4 leaf[THREADS];          // a0, c0, a1, first index of the lane's triangles in the warp's list
+  const float4* tri[THREADS];
+  unsigned char own[THREADS / 32][kOccOwn];
 };
+using OccExchange = OccExchangeT<128>;
 
 // Phase 2 (all 32 lanes): the pending leaves' triangles, 32 at a time;
 // true for a lane whose ray has a hit at tmin < t < aim. Clears the pending
 // leaves. SAME_TRI: one scene for the whole warp (its triangle array is not
 // exchanged).
-template <bool SAME_TRI, class Stack>
+template <bool SAME_TRI, class Stack, int THREADS>
 RMN_D bool occ_leaves(const float4* __restrict__ tri, const TRay& r, float tmin, float aim, OccT<Stack>& t,
-                      OccExchange& x) {
+                      OccExchangeT<THREADS>& x) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const int wb = threadIdx.x & ~31;
-  unsigned char* own = x.own[threadIdx.x >> 5];
+  const int me = THREADS == 32 ? lane : (int)threadIdx.x;  // this lane's place in the exchange
+  const int wb = me & ~31;
+  unsigned char* own = x.own[me >> 5];
   const int cnt = t.c0 + t.c1;  // at most 30
   if (!__any_sync(FULL, cnt > 0)) return false;
   int incl = cnt;
@@ -568,10 +572,10 @@ RMN_D bool occ_leaves(const float4* __restrict__ tri, const TRay& r, float tmin,
   const int total = __shfl_sync(FULL, incl, 31);  // at most kOccOwn
   const int excl = incl - cnt;
   if (cnt > 0) {
-    x.ray[2 * threadIdx.x] = make_float4(r.o.x, r.o.y, r.o.z, aim);
-    x.ray[2 * threadIdx.x + 1] = make_float4(r.d.x, r.d.y, r.d.z, tmin);
-    x.leaf[threadIdx.x] = make_int4(t.a0, t.c0, t.a1, excl);
-    if (!SAME_TRI) x.tri[threadIdx.x] = tri;
+    x.ray[2 * me] = make_float4(r.o.x, r.o.y, r.o.z, aim);
+    x.ray[2 * me + 1] = make_float4(r.d.x, r.d.y, r.d.z, tmin);
+    x.leaf[me] = make_int4(t.a0, t.c0, t.a1, excl);
+    if (!SAME_TRI) x.tri[me] = tri;
     for (int k = excl; k < incl; ++k) own[k] = (unsigned char)lane;
   }
   __syncwarp();
