@@ -25,7 +25,7 @@
 //    (depth bits, index): each tile ranks its own pixels on the device. A
 //    NaN depth (a pixel without a hit) compares false both ways in the
 //    reference's comparator, so its place depends on std::stable_sort's
-//    algorithm: then the host runs that very sort and the key is the rank.
+//    algorithm, which stable_order.cu carries out; the key is then the rank.
 //    A plan (order, radii, weights) serves every blur of the same G-buffer.
 #include <algorithm>
 #include <cmath>
@@ -267,19 +267,21 @@ __global__ void dof_source_kernel(const float* __restrict__ depth, float coc, fl
 
 // Tile t = (tx, ty) of a T-grid covers x in [tx T, min(W, tx T + T)) and
 // likewise y; its list occupies [tile_start[t], tile_start[t + 1]).
-__global__ void dof_rank_kernel(const float* __restrict__ depth, const int* __restrict__ tile_start, int W, int H,
+// `order`: the high word of a pixel's key -- its depth's bits, or (NaN depths)
+// its rank in the sorted order.
+__global__ void dof_rank_kernel(const unsigned* __restrict__ order, const int* __restrict__ tile_start, int W, int H,
                                 int T, int TW, unsigned long long* __restrict__ key, int* __restrict__ pix) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
   if (x >= W) return;
   const int tx = x / T, ty = y / T;
   const int x0 = tx * T, y0 = ty * T, x1 = min(W, x0 + T), y1 = min(H, y0 + T);
   const int p = y * W + x;
-  const unsigned long long kp = ((unsigned long long)__float_as_uint(depth[p]) << 32) | (unsigned)p;
+  const unsigned long long kp = ((unsigned long long)order[p] << 32) | (unsigned)p;
   int rank = 0;
   for (int qy = y0; qy < y1; ++qy)
     for (int qx = x0; qx < x1; ++qx) {
       const int q = qy * W + qx;
-      const unsigned long long kq = ((unsigned long long)__float_as_uint(depth[q]) << 32) | (unsigned)q;
+      const unsigned long long kq = ((unsigned long long)order[q] << 32) | (unsigned)q;
       rank += kq < kp ? 1 : 0;
     }
   const int slot = tile_start[ty * TW + tx] + rank;
@@ -572,38 +574,16 @@ cudaError_t dof_plan_create(const float* gbuf, int W, int H, float focus, float 
   p->tile_start = static_cast<int*>(alloc(sizeof(int) * tile_start.size()));
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(p->tile_start, tile_start.data(), sizeof(int) * tile_start.size(), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess && !hflags[0]) {
-    dof_rank_kernel<<<row_grid(W, H), 128, 0, st>>>(depth, p->tile_start, W, H, p->T, p->TW, p->key, p->pix);
+  const unsigned* order = reinterpret_cast<const unsigned*>(depth);  // non-negative: their bits ascend with them
+  if (e == cudaSuccess && hflags[0]) {
+    // NaN depths: the order the reference's std::stable_sort gives them
+    unsigned* rank = static_cast<unsigned*>(alloc(sizeof(unsigned) * n));
+    if (e == cudaSuccess) e = rmn::launch_stable_order(depth, n, rank, st);
+    order = rank;
+  }
+  if (e == cudaSuccess) {
+    dof_rank_kernel<<<row_grid(W, H), 128, 0, st>>>(order, p->tile_start, W, H, p->T, p->TW, p->key, p->pix);
     e = cudaGetLastError();
-  } else if (e == cudaSuccess) {
-    // NaN depths: the reference's own std::stable_sort decides the order
-    std::vector<float> hd(n);
-    e = cudaMemcpyAsync(hd.data(), depth, sizeof(float) * n, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) {
-      struct PixelPos {
-        int x, y;
-        float depth;
-      };
-      std::vector<PixelPos> pixs;
-      pixs.reserve(n);
-      for (int y = 0; y < H; ++y)
-        for (int x = 0; x < W; ++x) pixs.push_back({x, y, hd[(size_t)y * W + x]});
-      std::stable_sort(pixs.begin(), pixs.end(),
-                       [](const PixelPos& a, const PixelPos& b) { return a.depth < b.depth; });
-      std::vector<unsigned long long> hkey(n);
-      std::vector<int> hpix(n);
-      std::vector<int> fill(tile_start.begin(), tile_start.end() - 1);
-      for (int r = 0; r < n; ++r) {  // ranks ascend within each tile
-        const PixelPos& q = pixs[r];
-        const int slot = fill[(size_t)(q.y / p->T) * p->TW + q.x / p->T]++;
-        hkey[slot] = (unsigned long long)r;
-        hpix[slot] = q.y * W + q.x;
-      }
-      e = cudaMemcpyAsync(p->key, hkey.data(), sizeof(unsigned long long) * n, cudaMemcpyHostToDevice, st);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(p->pix, hpix.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the host vectors go out of scope
-    }
   }
   // candidate lists: capacity of tile t = the pixels of its 3 x 3 tiles
   const size_t ntiles = (size_t)p->TW * p->TH;

@@ -186,6 +186,9 @@ cudaError_t dof_plan_create(const float* gbuf, int w, int h, float focus, float 
                             cudaStream_t st, DofPlan** out);
 cudaError_t dof_apply(const DofPlan* plan, float* rgb, cudaStream_t st);
 void dof_plan_destroy(DofPlan* plan, cudaStream_t st);
+// rank[p] = place of pixel p in the order std::stable_sort by depth gives,
+// NaN depths included (stable_order.cu).
+cudaError_t launch_stable_order(const float* depth, int n, unsigned* rank, cudaStream_t st);
 cudaError_t launch_gamma(float* rgb, int n, cudaStream_t st);
 cudaError_t launch_compose(const float* dd, const float* ds, const float* id, const float* is, const float* gbuf,
                            int w, int h, float exposure, int options, float* rgb, cudaStream_t stream);

@@ -1,0 +1,31 @@
+"""The depth order of the depth-of-field blur with NaN depths (pixels without
+a hit): csrc/stable_order.cu against the oracle, which runs std::stable_sort."""
+import numpy as np
+import pytest
+
+pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from raym0nade_gb300 import api  # noqa: E402
+from tests.golden.make_golden import PHOTO_POST, photo_records  # noqa: E402
+from tests.test_gpu_post import np_, photo_from_records  # noqa: E402
+
+
+# sizes about a chunk of 7, a half of one tile of 1792 and several merge
+# levels, odd (the last merge from the back) and even
+@pytest.mark.parametrize("w,h", [(1, 1), (2, 1), (3, 1), (7, 1), (5, 3), (64, 56), (61, 59), (128, 61), (97, 151)])
+@pytest.mark.parametrize("nan", ["some", "top", "bottom", "bands", "all"])
+def test_nan_depth_order(port, w, h, nan):
+    rec = photo_records(w, h, 31 + w)
+    r = rec.reshape(-1, 40)
+    n = w * h
+    i = np.arange(n)
+    miss = {"some": np.random.default_rng(w).random(n) < 0.3, "top": i < 0.4 * n, "bottom": i >= 0.6 * n,
+            "bands": (i // 13) % 3 == 0, "all": i >= 0}[nan]
+    r[:, 22:25] = np.round(r[:, 22:25] * 8) / 8  # ties
+    r[miss, 22:25] = np.nan
+    post = dict(PHOTO_POST, coc=9.0)
+    ph = photo_from_records(rec, post)
+    got = np_(ph.post_process(api.Full | api.DoDepthFieldBlur))
+    _, want = port.photo(rec, 8, api.Full | api.DoDepthFieldBlur, **post)
+    assert np.array_equal(got, want, equal_nan=True)
