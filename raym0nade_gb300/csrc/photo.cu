@@ -114,62 +114,109 @@ __global__ void filter_var_kernel(Bufs in, Bufs out, int W, int H) {
   out.b[z][i] = make_float4(p.x, p.y, p.z, V + E2 - dot3(E, E));
 }
 
-// getWeight, src/image.cpp:110-158 (sigma_z = sigma_l = sigma_m = 1,
-// sigma_n = 1024, eps 1e-2, eps_r 4e-2; every pixel's specular is the
-// HitInfo default 0.04, so its difference is 0).
-__device__ __forceinline__ float edge_weight(const float4* __restrict__ guide, size_t ip, size_t iq, float4 Lp,
-                                             float4 Lq, bool specular) {
-  const float4 q0 = guide[3 * iq], q1 = guide[3 * iq + 1];
-  if (!any_finite3(xyz(q0))) return 0.0f;
-  const float4 p0 = guide[3 * ip], p1 = guide[3 * ip + 1], p2 = guide[3 * ip + 2];
-  const float d = dot3(xyz(p1), xyz(q1));
-  float w = powf(0.0f < d ? d : 0.0f, 1024.0f);
-  if (w < 1e-6f) return 0.0f;
-  float k = 0.0f;
-  const float3 dir = norm3(xyz(q0) - xyz(p0));
-  const float st = fabsf(dot3(xyz(p2), dir));
-  const float tt = st / (sqrtf(1.0f - st * st) + RMN_EPS);
-  k += -tt / 1.0f;
-  const float rd = len3(xyz(Lp) - xyz(Lq)) / (1.0f * sqrtf(Lp.w) + 1e-2f);
-  k += -rd;
-  const float md = len3(f3(p0.w - q0.w, 0.04f - 0.04f, p1.w - q1.w));
-  k += -md / 1.0f;
-  if (k < -7.5f) return 0.0f;
-  w *= expf(k);
-  if (specular) w *= p2.w < 4e-2f ? 4e-2f : p2.w;
-  if (!isfinite(w)) return 0.0f;
-  return w;
-}
+// filterRadiance(..., step), src/image.cpp:160-199, with getWeight
+// (:110-158; sigma_z = sigma_l = sigma_m = 1, sigma_n = 1024, eps 1e-2,
+// eps_r 4e-2; every pixel's specular is the HitInfo default 0.04, so its
+// difference is 0).
+//
+// A thread filters one pixel of all four buffers: of a tap's weight only the
+// radiance term and the specular buffers' roughness factor differ between
+// them, while the normal term (powf), the plane distance (a normalisation, a
+// square root and three divisions) and the material term are the geometry's.
+// The pass is bound by instruction issue; a thread per pixel and buffer
+// computed the geometry's part four times. 1920x1080, a pass: 1.09 ms before,
+// 0.6 ms with all four; 6 blocks per SM (80 registers) against the 94 it would
+// take: another 0.05 ms less.
+__constant__ float c_h5[5] = {0.0625f, 0.25f, 0.375f, 0.25f, 0.0625f};
 
-// filterRadiance(..., step), src/image.cpp:160-199.
-__global__ void filter_pass_kernel(Bufs in, Bufs out, const float4* __restrict__ guide, int W, int H, int step) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
-  if (x >= W) return;
-  const float h[5] = {0.0625f, 0.25f, 0.375f, 0.25f, 0.0625f};
-  const bool specular = (z & 1) != 0;  // Ds, Is
-  const float4* r = in.b[z];
+__global__ void __launch_bounds__(128, 6) filter_pass_kernel(Bufs in, Bufs out, const float4* __restrict__ guide, int W,
+                                                          int H, int step) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+  if (x >= W || y >= H) return;
   const size_t i = (size_t)y * W + x;
-  float3 rb = f3(0.0f);
-  float vb = 0.0f;
-  if (any_finite3(xyz(guide[3 * i]))) {
-    const float4 Lp = r[i];
-    float ws = 0.0f;
-    for (int dy = -2; dy <= 2; ++dy)
-      for (int dx = -2; dx <= 2; ++dx) {
-        int nx = x + dx * step, ny = y + dy * step;
-        if (nx < 0 || nx >= W || ny < 0 || ny >= H) continue;
-        float wt = h[dx + 2] * h[dy + 2];
-        const size_t j = (size_t)ny * W + nx;
-        const float4 Lq = r[j];
-        if (dx != 0 || dy != 0) wt *= edge_weight(guide, i, j, Lp, Lq, specular);
-        ws += wt;
-        rb += xyz(Lq) * wt;
-        vb += Lq.w * wt * wt;
-      }
-    rb = rb / ws;
-    vb /= ws * ws;
+  float3 rb[4];
+  float vb[4];
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    rb[b] = f3(0.0f);
+    vb[b] = 0.0f;
   }
-  out.b[z][i] = make_float4(rb.x, rb.y, rb.z, vb);
+  const float4 p0 = guide[3 * i];
+  if (any_finite3(xyz(p0))) {
+    const float4 p1 = guide[3 * i + 1], p2 = guide[3 * i + 2];
+    const float rough = p2.w < 4e-2f ? 4e-2f : p2.w;
+    float3 Lp[4];
+    float ws[4], sl[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const float4 v = in.b[b][i];
+      Lp[b] = xyz(v);
+      sl[b] = 1.0f * sqrtf(v.w) + 1e-2f;
+      ws[b] = 0.0f;
+    }
+#pragma unroll 1
+    for (int dy = -2; dy <= 2; ++dy) {
+      const int ny = y + dy * step;
+      if (ny < 0 || ny >= H) continue;
+#pragma unroll 1
+      for (int dx = -2; dx <= 2; ++dx) {
+        const int nx = x + dx * step;
+        if (nx < 0 || nx >= W) continue;
+        const float hh = c_h5[dx + 2] * c_h5[dy + 2];
+        const size_t j = (size_t)ny * W + nx;
+        const bool centre = dx == 0 && dy == 0;
+        float4 Lq[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) Lq[b] = in.b[b][j];
+        // the geometry's part: w, and k before and after the radiance term
+        float w = 0.0f, tt = 0.0f, md = 0.0f;
+        if (!centre) {
+          const float4 q0 = guide[3 * j], q1 = guide[3 * j + 1];
+          if (any_finite3(xyz(q0))) {
+            const float d = dot3(xyz(p1), xyz(q1));
+            w = powf(0.0f < d ? d : 0.0f, 1024.0f);
+            if (w < 1e-6f) {
+              w = 0.0f;
+            } else {
+              const float3 dir = norm3(xyz(q0) - xyz(p0));
+              const float st = fabsf(dot3(xyz(p2), dir));
+              tt = st / (sqrtf(1.0f - st * st) + RMN_EPS);
+              md = len3(f3(p0.w - q0.w, 0.04f - 0.04f, p1.w - q1.w));
+            }
+          }
+        }
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          float wt = hh;
+          if (!centre) {
+            float e = 0.0f;
+            if (w != 0.0f) {  // a NaN goes on and is dropped below
+              float k = 0.0f;
+              k += -tt / 1.0f;
+              k += -(len3(Lp[b] - xyz(Lq[b])) / sl[b]);
+              k += -md / 1.0f;
+              if (!(k < -7.5f)) {
+                e = w * expf(k);
+                if (b & 1) e *= rough;  // Ds, Is
+                if (!isfinite(e)) e = 0.0f;
+              }
+            }
+            wt *= e;
+          }
+          ws[b] += wt;
+          rb[b] += xyz(Lq[b]) * wt;
+          vb[b] += Lq[b].w * wt * wt;
+        }
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      rb[b] = rb[b] / ws[b];
+      vb[b] /= ws[b] * ws[b];
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < 4; ++b) out.b[b][i] = make_float4(rb[b].x, rb[b].y, rb[b].z, vb[b]);
 }
 
 // --------------------------------------------------------------- bloom ----
@@ -485,8 +532,9 @@ cudaError_t launch_filter(float* const bufs[4], const float* gbuf, int W, int H,
   // passes of step 1, 2, 4, 8, 16: B -> A -> B -> A -> B -> A
   bool toA = true;
   for (int step = 1; step <= 16; step *= 2) {
-    if (toA) filter_pass_kernel<<<row_grid(W, H, 4), 128, 0, st>>>(B, A, guide, W, H, step);
-    else filter_pass_kernel<<<row_grid(W, H, 4), 128, 0, st>>>(A, B, guide, W, H, step);
+    const dim3 grid((W + 31) / 32, (H + 3) / 4), block(32, 4);
+    if (toA) filter_pass_kernel<<<grid, block, 0, st>>>(B, A, guide, W, H, step);
+    else filter_pass_kernel<<<grid, block, 0, st>>>(A, B, guide, W, H, step);
     toA = !toA;
   }
   return cudaGetLastError();
