@@ -430,41 +430,116 @@ __global__ void __launch_bounds__(kCandThreads) dof_candidates_kernel(
   if (threadIdx.x == 0) cand_count[t] = filled;
 }
 
-// The receiving pixel (x, y): its tile's candidates, in order.
-__global__ void dof_fold_kernel(const float* __restrict__ rgb, const float4* __restrict__ src,
-                                const long long* __restrict__ cand_off, const int* __restrict__ cand,
-                                const int* __restrict__ cand_count, int W, int H, int T, int TW,
-                                float* __restrict__ out) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= W || y >= H) return;
-  const int t = (y / T) * TW + x / T;
+// The receivers of a tile: its candidates folded in order, for one image or
+// two at once (the weights are the plan's alone). A warp has 8 x 4 receivers;
+// a block stages the tile's candidates in shared memory, kFoldChunk at a time,
+// and each warp goes through those whose square of half-width radius touches
+// its 32 receivers: a lane tests one candidate, a vote makes the list, in
+// order. Positions are relative to the tile (at most 3 x 96 a side: exact in
+// float, as are their squares).
+//
+// The reference's tests of a pair, |dx| <= int(sqrt(c0^2 - dy^2)) and the
+// weight min(1, c0 - sqrt(dx^2 + dy^2)) / total, need neither root nor division
+// where the pair lies clearly inside: dx^2 <= c0^2 - dy^2 as floats makes the
+// root at least |dx| (the integer's square is exact and the root's rounding
+// monotone), and dx^2 + dy^2 < (c0 - 1)^2 (1 - 1e-6) makes c0 less the root at
+// least 1 (the margin is above the three roundings), so that the weight is
+// 1 / total, found once per candidate. What lies below 1 - 1e-6 times the
+// square is outside; the rest takes the reference's operations.
+//
+// A receiver that has gained so much that no weight of at least eps can be
+// added any more (0.99 - gained below eps / 2; a candidate's weight is at least
+// eps or skipped, and what is left of it after the cap is below eps, so it is
+// skipped) is done, and a block whose receivers are all done stops.
+constexpr int kFoldThreads = 256;
+constexpr int kFoldChunk = 128;
+
+template <int NI>
+__global__ void __launch_bounds__(kFoldThreads) dof_fold_kernel(
+    const float* __restrict__ in0, const float* __restrict__ in1, const float4* __restrict__ src,
+    const long long* __restrict__ cand_off, const int* __restrict__ cand, const int* __restrict__ cand_count, int W,
+    int H, int T, int TW, float* __restrict__ out0, float* __restrict__ out1) {
+  __shared__ float4 place[kFoldChunk];       // x, y, radius, c0
+  __shared__ float2 weight[kFoldChunk];      // the sender's total weight, (c0 - 1)^2 (1 - 1e-6) or 0
+  __shared__ float4 colour[NI][kFoldChunk];  // rgb, 1 / the total weight
+  const int t = blockIdx.x, lane = threadIdx.x & 31;
+  const int rect = (blockIdx.y * blockDim.x + threadIdx.x) >> 5, across = (T + 7) / 8;
+  const int x0 = (t % TW) * T, y0 = (t / TW) * T;
+  const int ex = (rect % across) * 8, ey = (rect / across) * 4;  // the warp's receivers in the tile
+  const int rx = ex + (lane & 7), ry = ey + (lane >> 3);
+  const bool receiver = rx < T && ry < T && x0 + rx < W && y0 + ry < H;
+  const float wx = (float)ex, wy = (float)ey, x = (float)rx, y = (float)ry;
   const int* c = cand + cand_off[t];
   const int n = cand_count[t];
-  float3 blur = f3(0.0f);
+  float3 blur[NI];
   float gained = 0.0f;
-  for (int k = 0; k < n; ++k) {
-    const int s = c[k];
-    const int sx = s % W, sy = s / W;
-    const int dx = x - sx, dy = y - sy;
-    const float4 sv = src[s];
-    const int radius = __float_as_int(sv.z);
-    if (dy < -radius || dy > radius) continue;
-    const float c0 = sv.x;
-    const int xlen = dof_int(sqrtf(c0 * c0 - (float)(dy * dy)));
-    if (dx < -xlen || dx > xlen) continue;
-    float w = c0 - sqrtf((float)(dx * dx + dy * dy));
-    w = (1.0f < w ? 1.0f : w) / sv.y;
-    if (w < RMN_EPS) continue;
-    if (gained + w > 0.99f) w = 0.99f - gained;
-    if (w < RMN_EPS) continue;
-    blur += f3(rgb[3 * (size_t)s], rgb[3 * (size_t)s + 1], rgb[3 * (size_t)s + 2]) * w;
-    gained += w;
+#pragma unroll
+  for (int m = 0; m < NI; ++m) blur[m] = f3(0.0f);
+  bool done = !receiver;
+  for (int k0 = 0; k0 < n; k0 += kFoldChunk) {
+    if (__syncthreads_and(done)) break;
+    const int len = min(kFoldChunk, n - k0);
+    for (int k = threadIdx.x; k < len; k += blockDim.x) {
+      const int s = c[k0 + k];
+      const float4 sv = src[s];
+      place[k] = make_float4((float)(s % W - x0), (float)(s / W - y0), (float)__float_as_int(sv.z), sv.x);
+      weight[k] = make_float2(sv.y, sv.x > 1.0f ? (sv.x - 1.0f) * (sv.x - 1.0f) * (1.0f - 1e-6f) : 0.0f);
+      const float inv = 1.0f / sv.y;
+      const size_t s3 = 3 * (size_t)s;
+      colour[0][k] = make_float4(in0[s3], in0[s3 + 1], in0[s3 + 2], inv);
+      if (NI > 1) colour[NI - 1][k] = make_float4(in1[s3], in1[s3 + 1], in1[s3 + 2], inv);
+    }
+    __syncthreads();
+    for (int kk = 0; kk < len; kk += 32) {
+      bool touches = false;
+      if (kk + lane < len) {
+        const float4 pl = place[kk + lane];
+        touches = pl.x + pl.z >= wx && pl.x - pl.z <= wx + 7.0f && pl.y + pl.z >= wy && pl.y - pl.z <= wy + 3.0f;
+      }
+      unsigned list = __ballot_sync(0xffffffffu, touches);
+      if (done) continue;
+      while (list) {
+        const int k = kk + __ffs(list) - 1;
+        list &= list - 1;
+        const float4 pl = place[k];
+        const float dx = x - pl.x, dy = y - pl.y, c0 = pl.w;
+        if (fabsf(dy) > pl.z || fabsf(dx) > pl.z) continue;  // the disc's half width is at most the radius
+        const float dx2 = dx * dx, dy2 = dy * dy, half2 = c0 * c0 - dy2;
+        if (!(dx2 <= half2)) {
+          if (half2 < dx2 * (1.0f - 1e-6f)) continue;
+          const float xlen = (float)dof_int(sqrtf(half2));
+          if (fabsf(dx) > xlen) continue;
+        }
+        float w;
+        if (dx2 + dy2 < weight[k].y) {
+          w = colour[0][k].w;
+        } else {
+          w = c0 - sqrtf(dx2 + dy2);
+          w = (1.0f < w ? 1.0f : w) / weight[k].x;
+        }
+        if (w < RMN_EPS) continue;
+        if (gained + w > 0.99f) w = 0.99f - gained;
+        if (w < RMN_EPS) continue;
+#pragma unroll
+        for (int m = 0; m < NI; ++m) {
+          const float4 v = colour[m][k];
+          blur[m] += f3(v.x, v.y, v.z) * w;
+        }
+        gained += w;
+      }
+      done = done || 0.99f - gained < 0.5f * RMN_EPS;
+    }
   }
-  const float3 o = blur / gained;
-  const size_t i = (size_t)y * W + x;
-  out[3 * i] = o.x;
-  out[3 * i + 1] = o.y;
-  out[3 * i + 2] = o.z;
+  if (!receiver) return;
+  const size_t i = (size_t)(y0 + ry) * W + x0 + rx;
+#pragma unroll
+  for (int m = 0; m < NI; ++m) {
+    const float3 o = blur[m] / gained;
+    float* out = m == 0 ? out0 : out1;
+    out[3 * i] = o.x;
+    out[3 * i + 1] = o.y;
+    out[3 * i + 2] = o.z;
+  }
 }
 
 __global__ void gamma_kernel(float* __restrict__ rgb, int n) {
@@ -671,12 +746,25 @@ cudaError_t dof_plan_create(const float* gbuf, int W, int H, float focus, float 
   return cudaSuccess;
 }
 
-// Photo::depthFeildBlur in place on rgb (device) with a plan of its G-buffer.
+// Photo::depthFeildBlur of in0 into out0 and, unless null, of in1 into out1,
+// with a plan of their G-buffer.
+cudaError_t dof_apply(const DofPlan* p, const float* in0, float* out0, const float* in1, float* out1,
+                      cudaStream_t st) {
+  const int per_tile = 32 * ((p->T + 7) / 8) * ((p->T + 3) / 4);  // 8 x 4 receivers a warp
+  const int threads = std::min(kFoldThreads, per_tile);
+  const dim3 grid((unsigned)(p->TW * p->TH), (per_tile + threads - 1) / threads);
+  if (in1)
+    dof_fold_kernel<2><<<grid, threads, 0, st>>>(in0, in1, p->src, p->cand_off, p->cand, p->cand_count, p->W, p->H,
+                                                 p->T, p->TW, out0, out1);
+  else
+    dof_fold_kernel<1><<<grid, threads, 0, st>>>(in0, nullptr, p->src, p->cand_off, p->cand, p->cand_count, p->W,
+                                                 p->H, p->T, p->TW, out0, nullptr);
+  return cudaGetLastError();
+}
+
+// The same in place on rgb.
 cudaError_t dof_apply(const DofPlan* p, float* rgb, cudaStream_t st) {
-  dim3 grid((p->W + 15) / 16, (p->H + 15) / 16), block(16, 16);
-  dof_fold_kernel<<<grid, block, 0, st>>>(rgb, p->src, p->cand_off, p->cand, p->cand_count, p->W, p->H, p->T, p->TW,
-                                          p->out);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = dof_apply(p, rgb, p->out, nullptr, nullptr, st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(rgb, p->out, sizeof(float) * 3 * (size_t)p->W * p->H, cudaMemcpyDeviceToDevice, st);
   return e;

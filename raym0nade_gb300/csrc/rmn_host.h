@@ -185,6 +185,8 @@ struct DofPlan;
 cudaError_t dof_plan_create(const float* gbuf, int w, int h, float focus, float coc, const float cam[3],
                             cudaStream_t st, DofPlan** out);
 cudaError_t dof_apply(const DofPlan* plan, float* rgb, cudaStream_t st);
+cudaError_t dof_apply(const DofPlan* plan, const float* in0, float* out0, const float* in1, float* out1,
+                      cudaStream_t st);
 void dof_plan_destroy(DofPlan* plan, cudaStream_t st);
 // rank[p] = place of pixel p in the order std::stable_sort by depth gives,
 // NaN depths included (stable_order.cu).
