@@ -235,9 +235,21 @@ __global__ void bloom_init_kernel(const float* __restrict__ rgb, float3* __restr
   bc[i] = b;
 }
 
-// One bloom pass: out = blur(in, step); rgb += out / 6.
-__global__ void bloom_pass_kernel(const float3* __restrict__ in, float3* __restrict__ out, float* __restrict__ rgb,
-                                  int W, int H, int step) {
+__device__ __forceinline__ float3 gamma3(float3 p) {  // Photo::gammaCorrection, src/image.cpp:454-468
+  p = max3(p, f3(0.0f));
+  const float c = lum3(p);
+  if (c > 0.75f) p = p / c * (tanhf(3.0f * (c - 0.75f)) / 3.0f + 0.75f);
+  p = min3(p, f3(1.0f));
+  const float e = 1.0f / 2.2f;
+  return f3(powf(p.x, e), powf(p.y, e), powf(p.z, e));
+}
+
+// One bloom pass: out = blur(in, step) (not kept by the LAST); rgb = base +
+// out / 6, gamma-corrected when the last pass is asked for it. base: the
+// image before bloom in the first pass, then rgb itself.
+template <bool LAST>
+__global__ void bloom_pass_kernel(const float3* __restrict__ in, float3* __restrict__ out, const float* base,
+                                  float* rgb, int W, int H, int step, bool gamma) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
   if (x >= W) return;
   const float h[5] = {0.0625f, 0.25f, 0.375f, 0.25f, 0.0625f};
@@ -249,11 +261,12 @@ __global__ void bloom_pass_kernel(const float3* __restrict__ in, float3* __restr
       col += in[(size_t)ny * W + nx] * h[ky + 2] * h[kx + 2];
     }
   const size_t i = (size_t)y * W + x;
-  out[i] = col;
-  const float3 a = col / 6.0f;
-  rgb[3 * i] += a.x;
-  rgb[3 * i + 1] += a.y;
-  rgb[3 * i + 2] += a.z;
+  if (!LAST) out[i] = col;
+  float3 p = f3(base[3 * i], base[3 * i + 1], base[3 * i + 2]) + col / 6.0f;
+  if (LAST && gamma) p = gamma3(p);
+  rgb[3 * i] = p.x;
+  rgb[3 * i + 1] = p.y;
+  rgb[3 * i + 2] = p.z;
 }
 
 // ----------------------------------------------------- depth of field -----
@@ -542,18 +555,13 @@ __global__ void __launch_bounds__(kFoldThreads) dof_fold_kernel(
   }
 }
 
-__global__ void gamma_kernel(float* __restrict__ rgb, int n) {
+__global__ void gamma_kernel(const float* in, float* out, int n) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float3 p = f3(rgb[3 * (size_t)i], rgb[3 * (size_t)i + 1], rgb[3 * (size_t)i + 2]);
-  p = max3(p, f3(0.0f));
-  const float c = lum3(p);
-  if (c > 0.75f) p = p / c * (tanhf(3.0f * (c - 0.75f)) / 3.0f + 0.75f);
-  p = min3(p, f3(1.0f));
-  const float e = 1.0f / 2.2f;
-  rgb[3 * (size_t)i] = powf(p.x, e);
-  rgb[3 * (size_t)i + 1] = powf(p.y, e);
-  rgb[3 * (size_t)i + 2] = powf(p.z, e);
+  const float3 p = gamma3(f3(in[3 * (size_t)i], in[3 * (size_t)i + 1], in[3 * (size_t)i + 2]));
+  out[3 * (size_t)i] = p.x;
+  out[3 * (size_t)i + 1] = p.y;
+  out[3 * (size_t)i + 2] = p.z;
 }
 
 struct DevScratch {
@@ -615,17 +623,20 @@ cudaError_t launch_filter(float* const bufs[4], const float* gbuf, int W, int H,
   return cudaGetLastError();
 }
 
-cudaError_t launch_bloom(float* rgb, int W, int H, cudaStream_t st) {
+// Photo::bloom of `in` into rgb (which may be `in`), then gammaCorrection when
+// asked for.
+cudaError_t launch_bloom(const float* in, float* rgb, int W, int H, bool gamma, cudaStream_t st) {
   const size_t n = (size_t)W * H;
   DevScratch sc{{}, st};
   float3* a = sc.get<float3>(n);
   float3* b = sc.get<float3>(n);
   if (sc.err != cudaSuccess) return sc.err;
-  bloom_init_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(rgb, a, (int)n);
-  for (int step = 1; step <= 16; step *= 2) {
-    bloom_pass_kernel<<<row_grid(W, H), 128, 0, st>>>(a, b, rgb, W, H, step);
+  bloom_init_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(in, a, (int)n);
+  for (int step = 1; step <= 8; step *= 2) {
+    bloom_pass_kernel<false><<<row_grid(W, H), 128, 0, st>>>(a, b, step == 1 ? in : rgb, rgb, W, H, step, false);
     std::swap(a, b);
   }
+  bloom_pass_kernel<true><<<row_grid(W, H), 128, 0, st>>>(a, b, rgb, rgb, W, H, 16, gamma);
   return cudaGetLastError();
 }
 
@@ -780,8 +791,9 @@ cudaError_t launch_dof(float* rgb, const float* gbuf, int W, int H, float focus,
   return e;
 }
 
-cudaError_t launch_gamma(float* rgb, int n, cudaStream_t st) {
-  gamma_kernel<<<(n + 255) / 256, 256, 0, st>>>(rgb, n);
+// Photo::gammaCorrection of n pixels; in == out allowed.
+cudaError_t launch_gamma(const float* in, float* out, int n, cudaStream_t st) {
+  gamma_kernel<<<(n + 255) / 256, 256, 0, st>>>(in, out, n);
   return cudaGetLastError();
 }
 

@@ -90,7 +90,8 @@ __device__ __forceinline__ float3 ld3(const float* p) { return f3(p[0], p[1], p[
 
 __global__ void compose_kernel(const float4* __restrict__ dd, const float4* __restrict__ ds,
                                const float4* __restrict__ id, const float4* __restrict__ is,
-                               const float* __restrict__ gbuf, int n, float exposure, int opt, float* __restrict__ rgb) {
+                               const float* __restrict__ gbuf, int n, float exposure, int opt, float* __restrict__ rgb,
+                               float* __restrict__ linear) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float* g = gbuf + (size_t)RMN_GBUFFER_FLOATS * i;
@@ -113,6 +114,11 @@ __global__ void compose_kernel(const float4* __restrict__ dd, const float4* __re
     float3 dc = (opt & RMN_SHADE_BASECOLOR) ? ld3(g) : f3(1.0f);
     p = dc * rd + rs;
     if (opt & RMN_SHADE_EMISSION) p += ld3(g + 3) * exposure;
+  }
+  if (linear) {
+    linear[3 * (size_t)i] = p.x;
+    linear[3 * (size_t)i + 1] = p.y;
+    linear[3 * (size_t)i + 2] = p.z;
   }
   if (opt & RMN_SHADE_GAMMA) {
     p = max3(p, f3(0.0f));
@@ -143,11 +149,12 @@ cudaError_t launch_fxaa(const float* in, float* out, int w, int h, cudaStream_t 
 }
 
 cudaError_t launch_compose(const float* dd, const float* ds, const float* id, const float* is, const float* gbuf,
-                           int w, int h, float exposure, int options, float* rgb, cudaStream_t stream) {
+                           int w, int h, float exposure, int options, float* rgb, cudaStream_t stream,
+                           float* linear) {
   int n = w * h;
   compose_kernel<<<(n + 255) / 256, 256, 0, stream>>>(
       reinterpret_cast<const float4*>(dd), reinterpret_cast<const float4*>(ds), reinterpret_cast<const float4*>(id),
-      reinterpret_cast<const float4*>(is), gbuf, n, exposure, options, rgb);
+      reinterpret_cast<const float4*>(is), gbuf, n, exposure, options, rgb, linear);
   return cudaGetLastError();
 }
 

@@ -177,7 +177,7 @@ cudaError_t launch_fxaa(const float* in, float* out, int w, int h, cudaStream_t 
 // Post passes (photo.cu); bufs = Dd, Ds, Id, Is (4 floats per pixel).
 cudaError_t launch_spatial_clamp(float* const bufs[4], int w, int h, cudaStream_t st);
 cudaError_t launch_filter(float* const bufs[4], const float* gbuf, int w, int h, cudaStream_t st);
-cudaError_t launch_bloom(float* rgb, int w, int h, cudaStream_t st);
+cudaError_t launch_bloom(const float* in, float* rgb, int w, int h, bool gamma, cudaStream_t st);
 cudaError_t launch_dof(float* rgb, const float* gbuf, int w, int h, float focus, float coc, const float cam[3],
                        cudaStream_t st);
 // A depth-of-field plan serves every blur of the same G-buffer and camera.
@@ -191,8 +191,11 @@ void dof_plan_destroy(DofPlan* plan, cudaStream_t st);
 // rank[p] = place of pixel p in the order std::stable_sort by depth gives,
 // NaN depths included (stable_order.cu).
 cudaError_t launch_stable_order(const float* depth, int n, unsigned* rank, cudaStream_t st);
-cudaError_t launch_gamma(float* rgb, int n, cudaStream_t st);
+cudaError_t launch_gamma(const float* in, float* out, int n, cudaStream_t st);
+// Photo::shade(options) (with gammaCorrection) into rgb; `linear`, unless
+// null, also receives the image before gamma.
 cudaError_t launch_compose(const float* dd, const float* ds, const float* id, const float* is, const float* gbuf,
-                           int w, int h, float exposure, int options, float* rgb, cudaStream_t stream);
+                           int w, int h, float exposure, int options, float* rgb, cudaStream_t stream,
+                           float* linear = nullptr);
 
 }  // namespace rmn
