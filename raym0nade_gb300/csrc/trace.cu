@@ -11,20 +11,23 @@
 // warp-aggregated atomic), so a warp no longer waits for its longest ray
 // (Aila & Laine, "Understanding the efficiency of ray traversal on GPUs",
 // HPG 2009: persistent threads with dynamic ray fetch).
+#include <algorithm>
+
 #include "rmn_host.h"
 #include "trace.cuh"
 
 namespace {
 
 // STACK: shared stack entries (RMN_STACK_SMALL for trees that fit it: one
-// more block per SM).
+// more block per SM). use: lanes of a warp that take rays (the others help
+// with the leaves).
 template <bool SHADOW, int STACK>
 __global__ void __launch_bounds__(128, RMN_COOP_BLOCKS(STACK)) trace_kernel(DevScene s, const float4* __restrict__ rays, int64_t n,
                                                     float4* __restrict__ hits, uint8_t* __restrict__ occ,
-                                                    unsigned long long* __restrict__ next, int* status) {
+                                                    unsigned long long* __restrict__ next, int* status, int use) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  bool active = false, retired = false;
+  bool active = false, retired = lane >= use;
   int64_t i = 0;
   TRay r;
   float tmin = 0.0f, aim = 0.0f, restart = 0.0f;
@@ -96,10 +99,10 @@ template <int STACK>
 __global__ void __launch_bounds__(128, RMN_OCC_BLOCKS) occ_kernel(DevScene s, const float4* __restrict__ rays,
                                                                           int64_t n, uint8_t* __restrict__ occ,
                                                                           unsigned long long* __restrict__ next,
-                                                                          int* status) {
+                                                                          int* status, int use) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  bool active = false, retired = false;
+  bool active = false, retired = lane >= use;
   int64_t i = 0;
   TRay r;
   float aim = 0.0f;
@@ -155,10 +158,18 @@ void launch_kernel(const DevScene& s, const float4* rays, int64_t n, float4* hit
   const bool order_free = SHADOW && !s.has_alpha;
   int blocks = order_free ? persistent_blocks((const void*)occ_kernel<STACK>, threads)
                           : persistent_blocks((const void*)trace_kernel<SHADOW, STACK>, threads);
-  int64_t need = (n + threads - 1) / threads;
+  // the rays go over all the warps the device holds, `use` of a warp's lanes
+  // taking one each: a warp's time is its rays' divergent steps one after the
+  // other. With 32 rays a warp while most of the device is idle, 1000 rays of the
+  // 130 k-triangle terrain take 114 us a call against 90 with one, 100 of the
+  // 1 M soup 327 against 192; from 32 rays a warp on (155,648 in all) nothing
+  // changes.
+  const int64_t warps = (int64_t)blocks * (threads / 32);
+  const int use = (int)std::min<int64_t>(32, (n + warps - 1) / warps);
+  const int64_t need = (n + (int64_t)use * (threads / 32) - 1) / ((int64_t)use * (threads / 32));
   if (need < blocks) blocks = (int)need;
-  if (order_free) occ_kernel<STACK><<<blocks, threads, 0, stream>>>(s, rays, n, occ, next, status);
-  else trace_kernel<SHADOW, STACK><<<blocks, threads, 0, stream>>>(s, rays, n, hits, occ, next, status);
+  if (order_free) occ_kernel<STACK><<<blocks, threads, 0, stream>>>(s, rays, n, occ, next, status, use);
+  else trace_kernel<SHADOW, STACK><<<blocks, threads, 0, stream>>>(s, rays, n, hits, occ, next, status, use);
 }
 
 cudaError_t launch(bool shadow, const DevScene& s, const rmn_ray* rays, int64_t n, rmn_hit* hits, uint8_t* occ,

@@ -236,3 +236,17 @@ def test_compose_matches_oracle(port):
     np.testing.assert_allclose(disp, z["display"], rtol=2e-6, atol=1e-7)
     fx = p.shade(api.Full | api.GAMMA | api.DoFXAA).cpu().numpy()
     np.testing.assert_allclose(fx, port.fxaa(disp), rtol=2e-6, atol=1e-7)
+
+
+# ray counts about the lines of the rays-per-warp rule: one ray, one and two a
+# warp (4,864 warps on 152 SMs), a full device, one ray more
+@pytest.mark.parametrize("n", [1, 31, 33, 4863, 4865, 9729, 155647, 155649])
+def test_ray_counts(port, n):
+    sc = scenes.random_soup(2000, 9)
+    m, o = api.Model(sc), port.scene(sc)
+    rays = scenes.random_rays(n, 10)
+    face, t, _ = api.split_hits(m.rayHit(torch.from_numpy(rays).cuda()))
+    of, ot, _ = o.trace_closest(rays)
+    assert np.array_equal(face, of) and np.array_equal(t, ot)
+    rays = scenes.random_rays(n, 11, shadow=True)
+    assert np.array_equal(m.rayHit_test(torch.from_numpy(rays).cuda()).cpu().numpy(), o.trace_shadow(rays))
