@@ -32,6 +32,7 @@
 // luminance-clamp boundary, the firefly clamp of :532-547, the NEE switch at
 // P_RR < 0.9) are held as the forward took them: the forward's record of
 // the sample the firefly clamp dropped is skipped.
+#include <algorithm>
 #include <vector>
 
 #include "integrator.cuh"
@@ -137,18 +138,62 @@ struct PathAdj {
   float3 A_light, A_w0, dbase;
 };
 
-// stk: the thread's deferred-child stack in shared memory. A real call, as
-// are brdf_logd and demod_adj: inlined at each of their call sites they
-// multiplied the replay's code, and its warps stalled on instruction fetch.
-__device__ __noinline__ bool occluded(const DevScene& s, float3 pos, float3 dir, float aim, int* status,
-                                         int2* stk) {
-  float tm = aim + RMN_EPS;  // HitRecord(eps, aimDepth + eps), Model::rayHit_test
-  int st = trace_shared<true>(s, make_tray(pos, dir), RMN_EPS, tm, aim, stk);  // no textured scenes here
-  if (st == -2) {
-    atomicExch(status, 1);
-    return false;
+// One warp's share of the traversals' shared memory: the ordered search's
+// stack and leaf keys, or occlusion's stack of references and leaf exchange.
+union AdjTrav {
+  struct {
+    int2 stack[RMN_STACK * 32];
+    unsigned long long keys[32];
+  } closest;
+  struct {
+    int stack[RMN_STACK * 32];
+    OccExchangeT<32> x;
+  } occ;
+};
+
+// The warp's shadow rays (all 32 lanes; `go`: the lane has one): whether each
+// is occluded, as Model::rayHit_test (no alpha-tested scenes here). A real
+// call, as are brdf_logd and demod_adj: inlined at each of their call sites
+// they multiplied the replay's code, and its warps stalled on instruction
+// fetch.
+__device__ __noinline__ bool occluded(const DevScene& s, float3 pos, float3 dir, float aim, bool go, AdjTrav& sh,
+                                      int* status) {
+  OccT<SharedStackRefN<RMN_STACK, 32>> t;
+  t.stack.base = sh.occ.stack + (threadIdx.x & 31);
+  occ_begin(s.root, t);
+  TRay r;
+  if (go) r = make_tray(pos, dir);
+  bool active = go, answer = false;
+  while (__ballot_sync(0xffffffffu, active) != 0) {
+    const int st = occ_nodes<false>(s.nodes, r, RMN_EPS, aim + RMN_EPS, t, active, kOccSteps, nullptr);
+    const bool o = occ_leaves<true>(s.tri, r, RMN_EPS, aim, t, sh.occ.x);
+    if (!active || (st == 0 && !o)) continue;
+    if (st == -2) atomicExch(status, 1);
+    answer = o && st != -2;
+    active = false;
   }
-  return tm < aim;
+  return answer;
+}
+
+// The warp's closest-hit rays likewise: the leaf-order triangle or -1 (-2 on
+// stack overflow), and its distance in tmax.
+__device__ __noinline__ int closest(const DevScene& s, float3 pos, float3 dir, float& tmax, bool go, AdjTrav& sh) {
+  TravT<SharedStackN<RMN_STACK, 32>> t;
+  t.stack.base = sh.closest.stack + (threadIdx.x & 31);
+  trav_begin(s, t, INFINITY);
+  TRay r;
+  if (go) r = make_tray(pos, dir);
+  bool active = go;
+  int hit = -1;
+  while (__ballot_sync(0xffffffffu, active) != 0) {
+    int st = coop_nodes<false>(s.nodes, r, RMN_EPS, t, active, kCoopSteps, nullptr);
+    coop_leaves<false, true>(s.tri, r, RMN_EPS, 0.0f, t, true, sh.closest.keys);
+    if (!active || st == 0) continue;
+    hit = st == -2 ? -2 : t.hit;
+    active = false;
+  }
+  tmax = t.tmax;
+  return hit;
 }
 
 // Log-derivatives of a factor clamp64(brdf(V, L)) * k of surface sf.
@@ -165,209 +210,303 @@ struct Record {
   float3 l, q, lr;
 };
 
-__device__ void adjoint_slot(const AdjJob& J, int pixel, int j, GradSink& G, int* status, int2* stk) {
-  const Params& p = J.p;
-  const DevScene& s = J.s;
-  const float* gb = J.gbuf + (size_t)RMN_GBUFFER_FLOATS * pixel;
-  const float3 pos0 = f3(gb[6], gb[7], gb[8]);
-  if (!any_finite3(pos0)) return;  // a miss: sky only, no material
-  const int m0 = (int)gb[19];
-  const float E = p.exposure;
-  const float3 gpx = f3(J.dimg[3 * (size_t)pixel], J.dimg[3 * (size_t)pixel + 1], J.dimg[3 * (size_t)pixel + 2]);
-  // The first vertex as the forward shades it: the material's base colour
-  // with renderPixel's tweak (the G-buffer's copy is the composed one).
+// The first vertex of a pixel as the forward shades it: the material's base
+// colour with renderPixel's tweak (the G-buffer's copy is the composed one).
+__device__ __forceinline__ Surf first_vertex(const AdjJob& J, const float* gb) {
   Surf g = default_surf();
-  g.base = tweak_base(f3(__ldg(&s.mats[m0].base)));
+  g.id = (int)gb[19];
+  g.base = tweak_base(f3(__ldg(&J.s.mats[g.id].base)));
   g.emis = f3(gb[3], gb[4], gb[5]);
-  g.pos = pos0;
+  g.pos = f3(gb[6], gb[7], gb[8]);
   g.shapeN = f3(gb[9], gb[10], gb[11]);
   g.surfN = f3(gb[12], gb[13], gb[14]);
   g.roughness = gb[15];
   g.metallic = gb[16];
   g.opacity = gb[17];
   g.eta = gb[18];
-  g.id = m0;
-  const float3 sav = f3(gb[0], gb[1], gb[2]);
-  if (j == 0) G.add(m0, 4, E * dot3(gpx, g.emis));  // Photo::shade's emission * exposure
-  if (len3(g.emis) > 0.0f) return;
-  RmnRng rng = rmn_rng(p.seed, (uint32_t)pixel, (uint32_t)j);
+  return g;
+}
+__device__ __forceinline__ const float* gbuf_at(const AdjJob& J, int pixel) {
+  return J.gbuf + (size_t)RMN_GBUFFER_FLOATS * pixel;
+}
+__device__ __forceinline__ float3 dimg_at(const AdjJob& J, int pixel) {
+  return f3(J.dimg[3 * (size_t)pixel], J.dimg[3 * (size_t)pixel + 1], J.dimg[3 * (size_t)pixel + 2]);
+}
 
-  if (j < p.spp_d) {  // a light sample of the first vertex
-    const float3 Vd = -norm3(g.pos - p.pos);
-    float lwt[8];
-    float tot = 0.0f;
-    if (s.sky_w == 0 && !light_weights(s, g, Vd, lwt, tot)) return;
-    float3 dir;
-    float aim;
+// Both kernels: dynamic shared memory holds the block's gradient table (when
+// it fits), flushed to the double-precision sums at the end.
+__device__ __forceinline__ GradSink grad_begin(float* sg, double* gout, int nmats) {
+  const bool use_sh = nmats <= kSharedMats;
+  if (use_sh)
+    for (int i = threadIdx.x; i < nmats * kGradPerMat; i += blockDim.x) sg[i] = 0.0f;
+  __syncthreads();
+  return GradSink{sg, gout, use_sh};
+}
+__device__ __forceinline__ void grad_end(const GradSink& G, int nmats) {
+  __syncthreads();
+  if (!G.use_sh) return;
+  for (int i = threadIdx.x; i < nmats * kGradPerMat; i += blockDim.x)
+    if (G.sh[i] != 0.0f) atomicAdd(G.gl + i, (double)G.sh[i]);
+}
+
+// Both kernels run in one block per SM whose warps go through the phases of a
+// round together (barriers between them): the code of a round is far larger
+// than an SM's instruction caches, so warps in different phases each wait for
+// their own instructions (20 cycles of 25 a warp waited between two issues
+// while every warp went its own way: 6.9 ms a pass over the paths below;
+// 2.9 ms with the phases in step).
+constexpr int kPathThreads = 512;
+
+// The light-sample slots of the first vertices, slot-major: a warp replays one
+// slot of 32 neighbouring pixels.
+__global__ void __launch_bounds__(kPathThreads, 1)
+    adjoint_light_kernel(AdjJob J, long long total, int nmats, double* gout, int* status) {
+  extern __shared__ __align__(16) unsigned char path_shared[];
+  AdjTrav& sh = reinterpret_cast<AdjTrav*>(path_shared)[threadIdx.x >> 5];
+  GradSink G = grad_begin(reinterpret_cast<float*>(path_shared + sizeof(AdjTrav) * (kPathThreads / 32)), gout, nmats);
+  const Params& p = J.p;
+  const DevScene& s = J.s;
+  const long long npx = (long long)p.W * p.H;
+  for (long long t0 = (long long)blockIdx.x * kPathThreads; t0 < total; t0 += (long long)gridDim.x * kPathThreads) {
+    const long long t = t0 + threadIdx.x;
+    const int pixel = (int)(t % npx), j = (int)(t / npx);
+    const float* gb = gbuf_at(J, pixel);
+    bool go = t < total && any_finite3(f3(gb[6], gb[7], gb[8]));  // else a miss: sky only, no material
+    Surf g;
+    float3 Vd, dir;
+    float aim = 0.0f;
     LSample ls;
     int li = -1;
-    if (!light_gen(s, g, Vd, lwt, tot, p.spp_d, rng, dir, aim, ls, &li)) return;
-    if (occluded(s, g.pos, dir, aim, status, stk)) return;
-    DemodAdj d = demod_adj(g.base, sav, ls.bsdf, ls.light, ls.weight, gpx, E);
-    if (!finite1(d.S) || d.S == 0.0f) return;
+    if (go) {
+      g = first_vertex(J, gb);
+      if (j == 0) G.add(g.id, 4, p.exposure * dot3(dimg_at(J, pixel), g.emis));  // Photo::shade's emission * exposure
+      go = !(len3(g.emis) > 0.0f);
+    }
+    if (go) {
+      RmnRng rng = rmn_rng(p.seed, (uint32_t)pixel, (uint32_t)j);
+      Vd = -norm3(g.pos - p.pos);
+      float lwt[8];
+      float tot = 0.0f;
+      go = (s.sky_w != 0 || light_weights(s, g, Vd, lwt, tot)) &&
+           light_gen(s, g, Vd, lwt, tot, p.spp_d, rng, dir, aim, ls, &li);
+    }
+    __syncthreads();
+    const bool occ = occluded(s, g.pos, dir, aim, go, sh, status);
+    __syncthreads();
+    if (occ || !go) continue;
+    DemodAdj d = demod_adj(g.base, f3(gb[0], gb[1], gb[2]), ls.bsdf, ls.light, ls.weight, dimg_at(J, pixel),
+                           p.exposure);
+    if (!finite1(d.S) || d.S == 0.0f) continue;
     float3 l, q, lr;
     brdf_logd(g, Vd, dir, 2, l, q, lr);
     const float3 A = d.df * ls.bsdf;
-    G.add_base(m0, A * l - d.S * q + d.dbase);
-    G.add(m0, 3, dot3(A, lr));
+    G.add_base(g.id, A * l - d.S * q + d.dbase);
+    G.add(g.id, 3, dot3(A, lr));
     if (li >= 0) G.add(__ldg(&s.lights[li].material), 4, d.S);
-    return;
   }
+  grad_end(G, nmats);
+}
 
-  // an indirect path
-  if (!(rng.next() < 1.0f)) return;
-  const float3 in = norm3(g.pos - p.pos);
-  Surf v0 = g;
-  v0.eta = 1.0f / v0.eta;
-  float3 dir, w0;
-  int f0 = 0;
-  ReflectAD ad0;
-  sample_reflect(v0, -in, rng, dir, w0, f0, &ad0);
-  if (!any_finite3(dir)) return;
-  float3 l0, q0, lr0;
-  brdf_logd(v0, -in, dir, ad0.clamped, l0, q0, lr0);
-  lr0 = lr0 + f3(ad0.score);
-  float paw = f0 > 0 ? 1.0f / (float)(1 + f0) : 1.0f;
-  float3 thr = f3(1.0f);
-  float rf = g.roughness;
-  int rfm = m0;
-  float3 o = g.pos;
-  int depth = 1;
-  bool exclude = true;
-  const int drop = J.dropped ? J.dropped[pixel] : -1;
-  const int sid0 = j * 8;
-  Record rec[kMaxRecords];
-  int nrec = 0;
+// The indirect paths. A lane replays one path at a time and takes the next
+// slot when it is done (slot-major, from one counter, once kRefill lanes of
+// the warp are free), so a warp does not wait for its longest path; each round
+// takes every lane's path over one vertex -- the bounce from the vertex it
+// stands at, first or later, the closest hit, its shading, and where the path
+// ends there its light samples -- so that lanes at different depths share every
+// call. The rays of a warp are traced together (coop_nodes / coop_leaves,
+// occ_nodes / occ_leaves).
+//
+// 512 threads of 128 registers: 256, 384, 768 and 1024 threads took 4.85, 4.13,
+// 4.01 and 4.48 ms a call where 512 took 3.88 (256x256, 32 spp, 16 materials;
+// the replay of one path per thread, without refill or cooperation, 6.40).
+constexpr int kRefill = 8;
+
+__global__ void __launch_bounds__(kPathThreads, 1)
+    adjoint_path_kernel(AdjJob J, long long total, int nmats, double* gout, unsigned long long* next, int* status) {
+  extern __shared__ __align__(16) unsigned char path_shared[];
+  const unsigned FULL = 0xffffffffu;
+  AdjTrav& sh = reinterpret_cast<AdjTrav*>(path_shared)[threadIdx.x >> 5];
+  float* sg = reinterpret_cast<float*>(path_shared + sizeof(AdjTrav) * (kPathThreads / 32));
+  const int lane = threadIdx.x & 31;
+  GradSink G = grad_begin(sg, gout, nmats);
+  const Params& p = J.p;
+  const DevScene& s = J.s;
+  const long long npx = (long long)p.W * p.H;
+  bool active = false, more = true;  // more: slots may be left (the same in every lane)
+  // the lane's path: rec[0] is its first vertex, rec[i] its i-th bounce
+  int pixel = 0, j = 0, depth = 0, rfm = 0, nrec = 0;
+  RmnRng rng;
+  Surf sf;  // the vertex the path stands at
+  float3 V, thr, w0;
+  float paw = 1.0f, rf = 0.0f, p_rr = 1.0f;
+  bool nee = false, exclude = true;
   PathAdj acc;
-  acc.S = 0.0f;
-  acc.A_light = acc.A_w0 = acc.dbase = f3(0.0f);
-  auto add_sample = [&](float3 light, float w) {
-    DemodAdj d = demod_adj(g.base, sav, w0, light, w, gpx, E);
-    if (!finite1(d.S) || d.S == 0.0f) {
-      d.S = 0.0f;
-      d.dlight = f3(0.0f);
-      return d;
-    }
-    acc.S += d.S;
-    acc.A_light += d.dlight * light;
-    acc.A_w0 += d.df * w0;
-    acc.dbase += d.dbase;
-    return d;
-  };
+  Record rec[kMaxRecords + 1];
   for (;;) {
-    float tm = INFINITY;
-    int h = trace_shared<false>(s, make_tray(o, dir), RMN_EPS, tm, 0.0f, stk);
-    if (h == -2) {
-      atomicExch(status, 1);
-      return;
-    }
-    if (h < 0) {
-      if (!exclude && s.sky_w && drop != sid0) add_sample(sky_get(s, dir) * thr, paw * p.inv_spp);
-      break;
-    }
-    Surf sf = default_surf();
-    sf.pos = o + dir * tm;
-    hit_info(s, h, dir, sf);
-    const int mk = sf.id;
-    const float own = sf.roughness;
-    const float rfn = fmaxf(rf, 1.0f * own);
-    const int am = own >= rf ? mk : rfm;
-    sf.roughness = fmaxf(sf.roughness, rfn);
-    rf = rfn;
-    rfm = am;
-    const float p_rr = 1.0f + (0.5f - 1.0f) * sqrtf(sf.roughness);
-    bool nee = p_rr < 0.9f;
-    if (len3(sf.emis) > RMN_EPS) {
-      if (!exclude && drop != sid0) {
-        DemodAdj d = add_sample(sf.emis * thr, paw * p.inv_spp);
-        G.add(mk, 4, d.S);
+    const unsigned idle = __ballot_sync(FULL, !active);
+    if (more && (__popc(idle) >= kRefill)) {
+      unsigned long long base = 0;
+      if (lane == 0) base = atomicAdd(next, (unsigned long long)__popc(idle));
+      base = __shfl_sync(FULL, base, 0);
+      more = (long long)base + __popc(idle) < total;
+      const long long t = (long long)base + __popc(idle & ((1u << lane) - 1u));
+      if (!active && t < total) {
+        pixel = (int)(t % npx);
+        j = p.spp_d + (int)(t / npx);
+        const float* gb = gbuf_at(J, pixel);
+        if (any_finite3(f3(gb[6], gb[7], gb[8]))) {  // else a miss: sky only, no material
+          sf = first_vertex(J, gb);
+          if (j == 0)  // Photo::shade's emission * exposure
+            G.add(sf.id, 4, p.exposure * dot3(dimg_at(J, pixel), sf.emis));
+          rng = rmn_rng(p.seed, (uint32_t)pixel, (uint32_t)j);
+          active = !(len3(sf.emis) > 0.0f) && rng.next() < 1.0f;
+          V = -norm3(sf.pos - p.pos);
+          rf = sf.roughness;
+          rfm = sf.id;
+          sf.eta = 1.0f / sf.eta;
+          depth = 0;
+          nrec = 0;
+          paw = 1.0f;
+          thr = f3(1.0f);
+          acc.S = 0.0f;
+          acc.A_light = acc.A_w0 = acc.dbase = f3(0.0f);
+        }
       }
-      break;
     }
-    if (!(rng.next() <= 1.0f)) break;
-    nee = nee && sf.entering;
-    const float3 V = -dir;
-    if (nee && (depth >= p.maxd || rng.next() > p_rr)) {
-      const int cnt = c_sample_count[depth < 16 ? depth : 16];
-      float k = 1.0f / 1.0f;
-      if (depth < p.maxd) k /= (1.0f - p_rr);
+    if (!__syncthreads_or(active || more)) break;
+    // the bounce from the vertex
+    float3 o = f3(0.0f), dir = f3(0.0f);
+    bool done = false;  // the path ends in this round
+    if (active) {
+      float3 wv;
+      int nf = 0;
+      ReflectAD ad;
+      sample_reflect(sf, V, rng, dir, wv, nf, &ad);
+      if (!any_finite3(dir) || (depth > 0 && depth == p.maxd)) {
+        active = false;  // nothing was added yet: a path's samples come at its end
+      } else {
+        Record& r = rec[nrec++];
+        r.m = sf.id;
+        r.a = rfm;
+        brdf_logd(sf, V, dir, ad.clamped, r.l, r.q, r.lr);
+        r.lr = r.lr + f3(ad.score);
+        if (depth == 0) {
+          w0 = wv;
+          paw = nf > 0 ? 1.0f / (float)(1 + nf) : 1.0f;
+        } else {
+          wv = wv / 1.0f;
+          if (nee) wv = wv / p_rr;
+          thr = thr * wv;
+          if (nf > 0) paw = paw * (1.0f / (float)(1 + nf));
+        }
+        exclude = depth == 0 || nee;
+        o = sf.pos;
+        depth++;
+      }
+    }
+    __syncthreads();
+    float tm;
+    const int h = closest(s, o, dir, tm, active, sh);
+    __syncthreads();
+    // one sample of the path: light, weight, into the path's sums
+    auto add_sample = [&](float3 light, float w) {
+      const float* gb = gbuf_at(J, pixel);
+      DemodAdj d = demod_adj(tweak_base(f3(__ldg(&s.mats[rec[0].m].base))), f3(gb[0], gb[1], gb[2]), w0, light, w,
+                             dimg_at(J, pixel), p.exposure);
+      if (!finite1(d.S) || d.S == 0.0f) {
+        d.S = 0.0f;
+        d.dlight = f3(0.0f);
+        return d;
+      }
+      acc.S += d.S;
+      acc.A_light += d.dlight * light;
+      acc.A_w0 += d.df * w0;
+      acc.dbase += d.dbase;
+      return d;
+    };
+    int cnt = 0;  // light samples of the vertex, where the path ends there
+    float kf = 1.0f;
+    if (active) {
+      const int drop = J.dropped ? J.dropped[pixel] : -1;
+      if (h == -2) {
+        atomicExch(status, 1);
+        active = false;
+      } else if (h < 0) {
+        if (!exclude && s.sky_w && drop != j * 8) add_sample(sky_get(s, dir) * thr, paw * p.inv_spp);
+        done = true;
+      } else {
+        sf = default_surf();
+        sf.pos = o + dir * tm;
+        hit_info(s, h, dir, sf);
+        const float own = sf.roughness;
+        const float rfn = fmaxf(rf, 1.0f * own);
+        if (own >= rf) rfm = sf.id;
+        sf.roughness = fmaxf(sf.roughness, rfn);
+        rf = rfn;
+        p_rr = 1.0f + (0.5f - 1.0f) * sqrtf(sf.roughness);
+        nee = p_rr < 0.9f;
+        V = -dir;
+        if (len3(sf.emis) > RMN_EPS) {
+          if (!exclude && drop != j * 8) {
+            DemodAdj d = add_sample(sf.emis * thr, paw * p.inv_spp);
+            G.add(sf.id, 4, d.S);
+          }
+          done = true;
+        } else if (!(rng.next() <= 1.0f)) {
+          done = true;
+        } else {
+          nee = nee && sf.entering;
+          if (nee && (depth >= p.maxd || rng.next() > p_rr)) {
+            cnt = c_sample_count[depth < 16 ? depth : 16];
+            if (depth < p.maxd) kf /= (1.0f - p_rr);
+            done = true;
+          }
+        }
+      }
+    }
+    // the light samples of the vertices where paths end
+    if (__syncthreads_or(cnt > 0)) {
       float lwt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       float tot = 0.0f;
-      if (s.sky_w == 0 && !light_weights(s, sf, V, lwt, tot)) break;
-      for (int n = 0; n < cnt; ++n) {
-        float3 ld;
-        float aim;
+      if (cnt > 0 && s.sky_w == 0 && !light_weights(s, sf, V, lwt, tot)) cnt = 0;
+      for (int n = 0; __syncthreads_or(n < cnt); ++n) {
+        float3 ld = f3(0.0f);
+        float aim = 0.0f;
         LSample ls;
         int li = -1;
-        if (!light_gen(s, sf, V, lwt, tot, cnt, rng, ld, aim, ls, &li)) continue;
-        ls.bsdf *= k;
-        if (occluded(s, sf.pos, ld, aim, status, stk)) continue;
-        if (drop == sid0 + n) continue;
+        const bool go = n < cnt && light_gen(s, sf, V, lwt, tot, cnt, rng, ld, aim, ls, &li);
+        __syncthreads();
+        const bool occ = occluded(s, sf.pos, ld, aim, go, sh, status);
+        __syncthreads();
+        if (occ || !go) continue;
+        if ((J.dropped ? J.dropped[pixel] : -1) == j * 8 + n) continue;
+        ls.bsdf *= kf;
         const float3 light = (ls.light * ls.bsdf) * thr;
         DemodAdj d = add_sample(light, ls.weight * paw * p.inv_spp);
         if (d.S == 0.0f) continue;
         float3 l, q, lr;
         brdf_logd(sf, V, ld, 2, l, q, lr);
         const float3 A = d.dlight * light;
-        G.add_base(mk, A * l - d.S * q);
-        G.add(am, 3, dot3(A, lr));
+        G.add_base(sf.id, A * l - d.S * q);
+        G.add(rfm, 3, dot3(A, lr));
         if (li >= 0) G.add(__ldg(&s.lights[li].material), 4, d.S);
       }
-      break;
     }
-    float3 nd, wv;
-    int nf = 0;
-    ReflectAD ad;
-    sample_reflect(sf, V, rng, nd, wv, nf, &ad);
-    wv = wv / 1.0f;
-    if (nee) wv = wv / p_rr;
-    if (!any_finite3(nd) || depth == p.maxd) break;
-    thr = thr * wv;
-    if (nrec < kMaxRecords) {
-      Record& r = rec[nrec++];
-      r.m = mk;
-      r.a = am;
-      brdf_logd(sf, V, nd, ad.clamped, r.l, r.q, r.lr);
-      r.lr = r.lr + f3(ad.score);
+    if (done) {
+      active = false;
+      if (acc.S != 0.0f) {
+        for (int i = 1; i < nrec; ++i) {
+          const Record& r = rec[i];
+          G.add_base(r.m, acc.A_light * r.l - acc.S * r.q);
+          G.add(r.a, 3, dot3(acc.A_light, r.lr));
+        }
+        const Record& r = rec[0];
+        G.add_base(r.m, acc.A_w0 * r.l - acc.S * r.q + acc.dbase);
+        G.add(r.m, 3, dot3(acc.A_w0, r.lr));
+      }
     }
-    if (nf > 0) paw = paw * (1.0f / (float)(1 + nf));
-    o = sf.pos;
-    dir = nd;
-    depth++;
-    exclude = nee;
   }
-  if (acc.S == 0.0f) return;
-  for (int i = 0; i < nrec; ++i) {
-    const Record& r = rec[i];
-    G.add_base(r.m, acc.A_light * r.l - acc.S * r.q);
-    G.add(r.a, 3, dot3(acc.A_light, r.lr));
-  }
-  G.add_base(m0, acc.A_w0 * l0 - acc.S * q0 + acc.dbase);
-  G.add(m0, 3, dot3(acc.A_w0, lr0));
-}
-
-__global__ void __launch_bounds__(128, 8) adjoint_kernel(AdjJob J, long long total, int nmats, double* gout,
-                                                      int* status) {
-  extern __shared__ float sg[];
-  const bool use_sh = nmats <= kSharedMats;
-  if (use_sh) {
-    for (int i = threadIdx.x; i < nmats * kGradPerMat; i += blockDim.x) sg[i] = 0.0f;
-    __syncthreads();
-  }
-  GradSink G{sg, gout, use_sh};
-  __shared__ int2 sstack[RMN_STACK * 128];  // traversal stacks (launched with 128 threads)
-  // Slot-major order: the lanes of a warp replay the same slot of 32
-  // neighbouring pixels, so they run the same kind of work (a first-vertex
-  // light sample or a path) on nearby surfaces.
-  const long long npx = (long long)J.p.W * J.p.H;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x)
-    adjoint_slot(J, (int)(t % npx), (int)(t / npx), G, status, sstack + threadIdx.x);
-  if (use_sh) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < nmats * kGradPerMat; i += blockDim.x)
-      if (sg[i] != 0.0f) atomicAdd(gout + i, (double)sg[i]);
-  }
+  grad_end(G, nmats);
 }
 
 __global__ void to_float_kernel(const double* in, float* out, int n) {
@@ -390,24 +529,34 @@ rmn_status launch_adjoint(const rmn_scene* scene, const rmn_render_args& args, c
   const int nmats = scene->dev.num_mats;
   const int ng = nmats * kGradPerMat;
   double* acc = nullptr;
-  int* status = nullptr;
   cudaError_t e = rmn::staging_malloc(reinterpret_cast<void**>(&acc), (size_t)ng * sizeof(double) + 16, st);
   if (e != cudaSuccess) return cuda_fail(e, "staging allocation (adjoint)");
-  status = reinterpret_cast<int*>(acc + ng);
+  unsigned long long* next = reinterpret_cast<unsigned long long*>(acc + ng);
+  int* status = reinterpret_cast<int*>(next + 1);
   e = cudaMemsetAsync(acc, 0, (size_t)ng * sizeof(double) + 16, st);
-  const long long total = (long long)J.p.W * J.p.H * J.p.slots;
-  const size_t smem = nmats <= kSharedMats ? (size_t)ng * sizeof(float) : 0;
-  int dev = 0, sms = 0, per_sm = 0;
+  const long long npx = (long long)J.p.W * J.p.H;
+  const long long lights = npx * J.p.spp_d, paths = npx * (J.p.slots - J.p.spp_d);
+  const size_t shared =
+      sizeof(AdjTrav) * (kPathThreads / 32) + (nmats <= kSharedMats ? (size_t)ng * sizeof(float) : 0);
+  int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adjoint_kernel, 128, smem);
-  if (per_sm < 1) per_sm = 1;
-  long long want = (total + 127) / 128;
-  long long grid = std::min<long long>(want, (long long)sms * per_sm * 8);
-  if (e == cudaSuccess && total > 0) {
-    adjoint_kernel<<<(unsigned)std::max<long long>(grid, 1), 128, smem, st>>>(J, total, nmats, acc, status);
-    e = cudaGetLastError();
+  // as many blocks as the device holds, or as the slots need
+  auto blocks = [&](const void* kernel, int threads, size_t shared, long long slots) {
+    int per_sm = 0;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, shared);
+    return (unsigned)std::min<long long>((slots + threads - 1) / threads, (long long)sms * std::max(per_sm, 1));
+  };
+  if (e == cudaSuccess && lights > 0) {
+    const unsigned g = blocks((const void*)adjoint_light_kernel, kPathThreads, shared, lights);
+    if (e == cudaSuccess) adjoint_light_kernel<<<g, kPathThreads, shared, st>>>(J, lights, nmats, acc, status);
   }
+  if (e == cudaSuccess && paths > 0) {
+    const unsigned g = blocks((const void*)adjoint_path_kernel, kPathThreads, shared, paths);
+    if (e == cudaSuccess) adjoint_path_kernel<<<g, kPathThreads, shared, st>>>(J, paths, nmats, acc, next, status);
+  }
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) {
     to_float_kernel<<<(ng + 127) / 128, 128, 0, st>>>(acc, dmat, ng);
     e = cudaGetLastError();
