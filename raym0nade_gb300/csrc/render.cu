@@ -1269,30 +1269,36 @@ __global__ void __launch_bounds__(128, RMN_OCC_BLOCKS) qocc_kernel(const Job* __
 
 // ------------------------------------------------- the wavefront in a block
 // block_kernel runs workers to the end of the render inside thread blocks:
-// each block owns up to kLocalWorkers of one lane's workers, keeps their
-// phases in queues in shared memory and fetches units until none is left. A
-// step of the block hands out tasks of up to 32 queue entries to its warps --
-// closest-hit rays with the shading of their answers, bounces, light samples
-// with their shadow rays, slot hand-offs, first bounces -- and every task
-// pushes what its workers do next into the queues of the following step. The
-// tasks run the logic kernels' own steps and traversals on the same records,
-// so the images are the wavefront's bit for bit.
+// each block -- one per SM -- owns up to kLocalWorkers of one lane's workers,
+// keeps their phases in queues in shared memory and fetches units until none is
+// left. A round of the block takes every path over one vertex, in three
+// stages: its rays are traced; their answers shaded and ended slots handed on;
+// the next rays made (bounces, first bounces, first-vertex light samples, one
+// light sample of every terminating vertex). The steps and traversals are the
+// logic kernels' own on the same records, so the images are the wavefront's bit
+// for bit.
 //
 // It takes the renders, and the ends of renders, that leave the wavefront
 // empty: an iteration of the wavefront costs 100-160 us however few workers
 // are left (nine launches in a row, each a chain of dependent loads 5-20 us
-// long), a step here 5-15 us, and a path needs about two steps a bounce.
+// long).
 //
-// 256 threads and 256 workers a block, 80 registers (sample_reflect and
-// light_gen spill below that) and about 72 KB of shared memory: three blocks
-// per SM. The stacks and leaf exchanges of the two traversals share one
-// piece of shared memory per warp, which runs one of them at a time.
-constexpr int kLocalThreads = 256;
-constexpr int kLocalWorkers = 256;
-constexpr int kLocalBlocks = 3;  // per SM
-enum LocalQueue { LQ_RAY = 0, LQ_NEE, LQ_PATH, LQ_BOUNCE, LQ_SLOT, LQ_WAIT, LQ_WORKER_QUEUES };
-enum LocalItems { LI_LIGHT = 0, LI_SHADOW, LI_QUEUES };  // worker * kDirectBatch + sample
-constexpr int kLocalKinds = LQ_WORKER_QUEUES + LI_QUEUES;
+// The kinds of work of a stage run one after the other, all warps on the same
+// kind: the steps' code is far larger than an SM's instruction caches, and with
+// tasks of all kinds side by side (three blocks of 256 threads per SM) a warp
+// waited 17 of 45 cycles between two issues for its instructions (Cornell
+// 256x256, 64 spp, all in this kernel: 12.9 ms against 4.5). Only when a stage
+// has no more tasks than the block has warps do they run side by side, cut to
+// fewer entries where that gives the idle warps work: then the longest of
+// them, not their sum, is what a round takes.
+// 512 threads keep 128 registers, which the steps need (sample_reflect and
+// light_gen spill below).
+constexpr int kLocalThreads = 512;
+constexpr int kLocalWorkers = 1024;
+// Kinds of work, by stage (two, two and four), each with a queue of workers or,
+// for LIGHT and SHADOW, of items (worker * kDirectBatch + sample). Those that
+// a round fills for the next one have two buffers.
+enum LocalKind { LK_RAY = 0, LK_SHADOW, LK_SHADE, LK_SLOT, LK_BOUNCE, LK_NEE, LK_PATH, LK_LIGHT, LK_COUNT };
 
 template <int STACK>
 union TravShared {  // of one warp
@@ -1309,10 +1315,11 @@ union TravShared {  // of one warp
 template <int STACK>
 struct LocalShared {
   TravShared<STACK> trav[kLocalThreads / 32];
-  uint16_t q[2][LQ_WORKER_QUEUES][kLocalWorkers];
-  uint16_t it[2][LI_QUEUES][kLocalWorkers * kDirectBatch];
-  int count[2][kLocalKinds];  // entries of q, then of it
-  int task;                   // next task of the step
+  int worker[kLocalWorkers];  // the workers behind the queues' entries
+  uint16_t ray[2][kLocalWorkers], slot[2][kLocalWorkers], nee[2][kLocalWorkers];
+  uint16_t bounce[kLocalWorkers], path[kLocalWorkers];
+  uint16_t shadow[2][kLocalWorkers * kDirectBatch], light[kLocalWorkers * kDirectBatch];
+  int count[2][LK_COUNT];  // by round parity; SHADE's is RAY's
 };
 
 // The lanes' closest-hit rays (all 32 lanes; `go`: the lane has worker w's):
@@ -1478,122 +1485,145 @@ RMN_D int nee_item(const Job* __restrict__ jobs, const Pool& P, int w, bool& mor
 }
 
 template <bool ALPHA, int STACK>
-__global__ void __launch_bounds__(kLocalThreads, kLocalBlocks)
+__global__ void __launch_bounds__(kLocalThreads, 1)
     block_kernel(const Job* __restrict__ jobs, int njobs, Pool P, Queues Q, const Ctl* __restrict__ ctl,
                  int per_block, unsigned long long* next_unit, long long total_units, float4* __restrict__ parts,
                  int* status) {
   extern __shared__ __align__(16) unsigned char local_shared[];
   LocalShared<STACK>& sh = *reinterpret_cast<LocalShared<STACK>*>(local_shared);
-  TravShared<STACK>& trav = sh.trav[threadIdx.x >> 5];
-  const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
+  constexpr int kWarps = kLocalThreads / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  TravShared<STACK>& trav = sh.trav[warp];
   // the workers waiting at the end of an iteration of parity 1, their rays
   // answered: worker[k] is the one behind the queues' entry k
-  __shared__ int worker[kLocalWorkers];
   const unsigned nc = ctl->q[1].c, nd = ctl->q[1].sd, nn = ctl->q[1].nw;
   const unsigned first = blockIdx.x * (unsigned)per_block;
-  if (threadIdx.x < 2 * kLocalKinds) (&sh.count[0][0])[threadIdx.x] = 0;
-  if (threadIdx.x == 0) sh.task = 0;
+  if (threadIdx.x < 2 * LK_COUNT) (&sh.count[0][0])[threadIdx.x] = 0;
   __syncthreads();
   int cur = 0;
-  // one atomic per lane: the lanes of a task push into different queues
-  auto push_worker = [&](int buf, int kind, int k) {
-    sh.q[buf][kind][atomicAdd(&sh.count[buf][kind], 1)] = (uint16_t)k;
-  };
-  auto push_lights = [&](int buf, int k, int n) {
-    const int at = atomicAdd(&sh.count[buf][LQ_WORKER_QUEUES + LI_LIGHT], n);
-    for (int j = 0; j < n; ++j) sh.it[buf][LI_LIGHT][at + j] = (uint16_t)(k * kDirectBatch + j);
-  };
-  // what follows a shading step
-  auto after_shade = [&](int buf, int k, int ph) {
-    if (ph == PH_WAIT_CLOSEST) push_worker(buf, LQ_RAY, k);
-    else if (ph == PH_NEE) push_worker(buf, LQ_NEE, k);
-    else if (ph == PH_BOUNCE) push_worker(buf, LQ_BOUNCE, k);
-    else push_worker(buf, LQ_SLOT, k);
-  };
+  // one atomic per lane: the lanes of a warp push into different queues
+  auto push = [&](uint16_t* q, int* count, int k) { q[atomicAdd(count, 1)] = (uint16_t)k; };
+  auto push_ray = [&](int buf, int k) { push(sh.ray[buf], &sh.count[buf][LK_RAY], k); };
+  auto push_slot = [&](int buf, int k) { push(sh.slot[buf], &sh.count[buf][LK_SLOT], k); };
   for (int k = threadIdx.x; k < per_block; k += kLocalThreads) {
     const unsigned i = first + k;
     if (i >= nc + nd + nn) break;
-    worker[k] = i < nc ? Q.c[1][i] : i - nc < nd ? Q.sd[1][i - nc] : Q.nw[1][i - nc - nd];
+    sh.worker[k] = i < nc ? Q.c[1][i] : i - nc < nd ? Q.sd[1][i - nc] : Q.nw[1][i - nc - nd];
     // an answered closest-hit ray is traced once more, to the same answer:
-    // its shading follows in that task
-    push_worker(cur, i < nc ? LQ_RAY : LQ_SLOT, k);
+    // its shading follows
+    if (i < nc) push_ray(cur, k);
+    else push_slot(cur, k);
   }
-  __syncthreads();
   unsigned long long unused = 0;
   for (;;) {
+    __syncthreads();
     int* count = sh.count[cur];
     const int nxt = cur ^ 1;
-    int total = 0;
-#pragma unroll
-    for (int kind = 0; kind < kLocalKinds; ++kind) total += (count[kind] + 31) >> 5;
-    if (total == 0) break;
-    for (;;) {
-      int task = 0;
-      if (lane == 0) task = atomicAdd(&sh.task, 1);
-      task = __shfl_sync(FULL, task, 0);
-      if (task >= total) break;
-      // the longest tasks first
-      int kind = LQ_RAY, at = task, n = count[LQ_RAY];
-      constexpr int order[kLocalKinds] = {LQ_RAY, LQ_WORKER_QUEUES + LI_LIGHT, LQ_NEE,
-                                          LQ_WORKER_QUEUES + LI_SHADOW, LQ_PATH, LQ_BOUNCE, LQ_SLOT, LQ_WAIT};
-#pragma unroll
-      for (int o = 0; o < kLocalKinds; ++o) {
-        kind = order[o];
-        n = count[kind];
-        const int tasks = (n + 31) >> 5;
-        if (at < tasks) break;
-        at -= tasks;
-      }
-      const int e = at * 32 + lane;
-      const bool go = e < n;
-      if (kind >= LQ_WORKER_QUEUES) {
-        const int item = go ? sh.it[cur][kind - LQ_WORKER_QUEUES][e] : 0;
-        const int k = item / kDirectBatch, j = item % kDirectBatch;
-        const int w = worker[k];
-        bool ray = go;
-        if (kind == LQ_WORKER_QUEUES + LI_LIGHT) {
-          ray = go && light_item(jobs, P, w, j);
-          // the worker's answers are there when this step ends
-          if (go && j == 0) push_worker(nxt, LQ_SLOT, k);
+    if (count[LK_RAY] + count[LK_SHADOW] + count[LK_SLOT] + count[LK_NEE] == 0) break;
+#pragma unroll 1
+    for (int stage = 0; stage < 3; ++stage) {
+      // the stage's kinds and their entries, read from shared memory wherever
+      // they are needed: kept in registers they would spill across the steps
+      const int k0 = 2 * stage, kinds = stage == 2 ? 4 : 2;
+      auto entries = [&](int q) { return count[k0 + q == LK_SHADE ? LK_RAY : k0 + q]; };
+      auto tasks_of = [&](int shift) {  // tasks of 1 << shift entries in the stage
+        int t = 0;
+        for (int q = 0; q < kinds; ++q) t += (entries(q) + (1 << shift) - 1) >> shift;
+        return t;
+      };
+      const bool together = tasks_of(5) <= kWarps;
+      int shift = 5;  // entries of a task
+      while (together && shift > 2 && tasks_of(shift - 1) <= kWarps) --shift;
+#pragma unroll 1
+      for (int pass = 0; pass < (together ? 1 : kinds); ++pass) {
+#pragma unroll 1
+        for (int task = warp;; task += kWarps) {
+          int q = pass, at = task;
+          if (together)
+            for (q = 0; q < kinds - 1; ++q) {
+              const int t = (entries(q) + (1 << shift) - 1) >> shift;
+              if (at < t) break;
+              at -= t;
+            }
+          const int nq = entries(q);
+          if ((at << shift) >= nq) break;
+          const int e = (at << shift) + lane;
+          const bool go = (lane >> shift) == 0 && e < nq;
+          switch (k0 + q) {
+            case LK_RAY: {
+              const int w = go ? sh.worker[sh.ray[cur][e]] : 0;
+              local_closest<ALPHA, STACK>(jobs, P, w, go, trav, status);
+              break;
+            }
+            case LK_SHADOW: {
+              const int item = go ? sh.shadow[cur][e] : 0, w = sh.worker[item / kDirectBatch];
+              local_shadow<ALPHA, STACK>(jobs, P, w, (size_t)w * kDirectBatch + item % kDirectBatch, go, trav, status);
+              break;
+            }
+            case LK_SHADE:
+              if (go) {
+                const int k = sh.ray[cur][e];
+                const int ph = shade_step(jobs, P, sh.worker[k], parts, status);
+                if (ph == PH_WAIT_CLOSEST) push_ray(nxt, k);
+                else if (ph == PH_NEE) push(sh.nee[cur], &count[LK_NEE], k);
+                else if (ph == PH_BOUNCE) push(sh.bounce, &count[LK_BOUNCE], k);
+                else push_slot(nxt, k);
+              }
+              break;
+            case LK_SLOT:  // with the answered light samples before the hand-off
+              if (go) {
+                const int k = sh.slot[cur][e], w = sh.worker[k];
+                if (worker_phase(P, w) == PH_WAIT_NEE) nee_emit_step(jobs, P, w, parts);
+                const int ph = slot_step(jobs, njobs, P, w, next_unit, total_units, parts);
+                if (ph == PH_PATH) {
+                  push(sh.path, &count[LK_PATH], k);
+                } else if (ph == PH_LIGHT) {
+                  const int c = light_batch(jobs, P, w), to = atomicAdd(&count[LK_LIGHT], c);
+                  for (int j = 0; j < c; ++j) sh.light[to + j] = (uint16_t)(k * kDirectBatch + j);
+                  push_slot(nxt, k);  // its samples are traced when the next round starts
+                }
+              }
+              break;
+            case LK_BOUNCE:
+              if (go) {
+                const int k = sh.bounce[e];
+                if (bounce_step(jobs, P, sh.worker[k]) == PH_WAIT_CLOSEST) push_ray(nxt, k);
+                else push_slot(nxt, k);
+              }
+              break;
+            case LK_NEE:
+              if (go) {
+                const int k = sh.nee[cur][e];
+                bool more;
+                const int j = nee_item(jobs, P, sh.worker[k], more);
+                if (j >= 0) push(sh.shadow[nxt], &sh.count[nxt][LK_SHADOW], k * kDirectBatch + j);
+                if (more) push(sh.nee[nxt], &sh.count[nxt][LK_NEE], k);
+                else push_slot(nxt, k);
+              }
+              break;
+            case LK_PATH:
+              if (go) {
+                const int k = sh.path[e];
+                if (path_step<false>(jobs, P, sh.worker[k], unused) == PH_WAIT_CLOSEST) push_ray(nxt, k);
+                else push_slot(nxt, k);
+              }
+              break;
+            default:  // LK_LIGHT
+              if (go) {
+                const int item = sh.light[e];
+                if (light_item(jobs, P, sh.worker[item / kDirectBatch], item % kDirectBatch))
+                  push(sh.shadow[nxt], &sh.count[nxt][LK_SHADOW], item);
+              }
+              break;
+          }
+          __syncwarp();
+          if (together) break;
         }
-        __syncwarp();
-        if (__any_sync(FULL, ray))
-          local_shadow<ALPHA, STACK>(jobs, P, w, (size_t)w * kDirectBatch + j, ray, trav, status);
-      } else {
-        const int k = go ? sh.q[cur][kind][e] : 0;
-        const int w = worker[k];
-        if (kind == LQ_RAY) {
-          local_closest<ALPHA, STACK>(jobs, P, w, go, trav, status);
-          if (go) after_shade(nxt, k, shade_step(jobs, P, w, parts, status));
-        } else if (!go) {
-        } else if (kind == LQ_BOUNCE) {
-          push_worker(nxt, bounce_step(jobs, P, w) == PH_WAIT_CLOSEST ? LQ_RAY : LQ_SLOT, k);
-        } else if (kind == LQ_PATH) {
-          push_worker(nxt, path_step<false>(jobs, P, w, unused) == PH_WAIT_CLOSEST ? LQ_RAY : LQ_SLOT, k);
-        } else if (kind == LQ_NEE) {
-          bool more;
-          const int j = nee_item(jobs, P, w, more);
-          if (j >= 0)
-            sh.it[nxt][LI_SHADOW][atomicAdd(&sh.count[nxt][LQ_WORKER_QUEUES + LI_SHADOW], 1)] =
-                (uint16_t)(k * kDirectBatch + j);
-          push_worker(nxt, more ? LQ_NEE : LQ_WAIT, k);
-        } else if (kind == LQ_SLOT) {
-          if (worker_phase(P, w) == PH_WAIT_NEE) nee_emit_step(jobs, P, w, parts);
-          const int ph = slot_step(jobs, njobs, P, w, next_unit, total_units, parts);
-          if (ph == PH_LIGHT) push_lights(nxt, k, light_batch(jobs, P, w));
-          else if (ph == PH_PATH) push_worker(nxt, LQ_PATH, k);
-        } else {  // LQ_WAIT: the worker's last shadow ray is traced in this step
-          push_worker(nxt, LQ_SLOT, k);
-        }
+        __syncthreads();
       }
-      __syncwarp();
     }
-    __syncthreads();  // the step's queues are read, its records written
-    if (threadIdx.x < kLocalKinds) sh.count[cur][threadIdx.x] = 0;
-    if (threadIdx.x == 0) sh.task = 0;
+    if (threadIdx.x < LK_COUNT) count[threadIdx.x] = 0;
     cur = nxt;
-    __syncthreads();
   }
 }
 
@@ -1945,15 +1975,19 @@ static cudaError_t launch_iteration(BatchState* b, int lane, cudaStream_t st, Co
   return cudaGetLastError();
 }
 
-// The workers that block_kernel holds on the device at once. A render of no
-// more units runs in it from the start, and a longer one ends in it once no
-// unit is left and no more workers live: below this line the wavefront's
-// kernels are mostly latency, above it block_kernel's blocks would queue up.
-// Measured (Cornell 160x90, 4 spp, 28,800 units: 0.87 ms against 2.1 ms with
-// two wavefront iterations first; 256x256, 16 spp, 328 k units: 3.8 against
-// 2.35; the glass box 250x250, 16 spp ended at 60-120 k workers: 9.3-9.7 ms, at
-// 250 k: 11.9).
-static long long block_capacity() { return (long long)device_sms() * kLocalBlocks * kLocalWorkers; }
+// The workers block_kernel holds on the device at once: a render ends in it
+// once no unit is left and no more workers than these live. (The end taken at
+// 60 k, 155,648 and 400 k workers: the glass box 250x250, 16 spp, 8.9, 8.4 and
+// 9.1 ms; Cornell 256x256, 64 spp, 4.3, 4.3 and 4.1; soup 400x300, 16 spp, 6.5,
+// 6.6 and 6.6; without block_kernel 10.8, 5.8 and 9.5.)
+static long long block_capacity() { return (long long)device_sms() * kLocalWorkers; }
+// A render of no more units runs in it from the start. Its workers fetch more
+// units as theirs end, but its blocks run fewer warps than the wavefront's
+// kernels: Cornell 256x256, 16 spp, 328 k units: 1.74 ms against 2.0 with the
+// wavefront first; the textured room 320x240, 8 spp, 230 k: 1.5 against 1.84; a
+// terrain 480x270, 16 spp, 648 k: 2.9 against 2.75; Cornell 64 spp, 1.05 M: 5.2
+// against 4.3.
+constexpr long long kDirectUnits = 400000;
 
 // block_kernel over the n workers of one lane that wait at the end of an
 // iteration of parity 1, or were seeded.
@@ -1963,7 +1997,7 @@ static cudaError_t launch_block(BatchState* b, int lane, long long n, cudaStream
   const int sms = device_sms();
   // one block per SM while its queues hold its share of the workers: fuller
   // queues make fuller tasks
-  const int per_block = (int)std::min<long long>(kLocalWorkers, std::max<long long>(64, (n + sms - 1) / sms));
+  const int per_block = (int)std::min<long long>(kLocalWorkers, std::max<long long>(32, (n + sms - 1) / sms));
   const unsigned grid = (unsigned)((n + per_block - 1) / per_block);
   Ctl* ctl = &b->d_ctl->lane[lane];
   cudaError_t e = cudaSuccess;
@@ -2246,8 +2280,11 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
     const size_t budget = free_device_bytes() / 4;
     while (per > 4096 && worker_bytes(glass, tex) * (size_t)per * b->lanes > budget) per /= 2;
   }
-  b->direct = b->table.total_units <= block_capacity();
-  if (b->direct) b->lanes = 1;
+  b->direct = b->table.total_units <= kDirectUnits;
+  if (b->direct) {
+    b->lanes = 1;
+    per = std::min(per, block_capacity());
+  }
   while (b->lanes > 1 && (long long)b->lanes * 128 > b->table.total_units) --b->lanes;
   per = std::min<long long>(per, (b->table.total_units + b->lanes - 1) / b->lanes);
   if (per < 1) per = 1;

@@ -25,11 +25,12 @@ def _case(name, w, h, spp, depth):
 
 
 # one unit, one worker, fewer workers than a block, an odd count over several
-# blocks, about the capacity of the device (116,736 units), and renders whose
-# wavefront runs first
+# blocks, about as many units as workers the device holds (155,648) and as the
+# kernel takes from the start (400,000), and renders whose wavefront runs first
 @pytest.mark.parametrize("name,w,h,spp,depth", [
     ("cornell", 1, 1, 1, 1), ("cornell", 1, 1, 2, 16), ("cornell", 33, 17, 5, 3), ("cornell", 97, 61, 9, 16),
-    ("cornell", 208, 187, 9, 8), ("cornell", 209, 187, 9, 8), ("cornell", 200, 150, 33, 16),
+    ("cornell", 240, 216, 9, 8), ("cornell", 241, 217, 9, 8), ("cornell", 365, 365, 9, 8),
+    ("cornell", 366, 366, 9, 8), ("cornell", 200, 150, 65, 16),
     ("glass", 5, 3, 1, 16), ("glass", 61, 47, 3, 16), ("glass", 90, 80, 16, 12),
     ("textured", 7, 5, 4, 16), ("textured", 120, 90, 8, 16), ("textured", 200, 160, 32, 8),
     ("terrain", 31, 29, 7, 16), ("terrain", 160, 90, 16, 16), ("terrain", 320, 200, 40, 16),
