@@ -358,8 +358,8 @@ __device__ __forceinline__ void push(int* q, unsigned int* qn, int w) { q[agg_in
 // list of the workers in its phase, so a warp executes one phase's code:
 //   shade_kernel  closest-hit answers (sampleRay's body): emit the sky or an
 //                 emitter, start the terminating vertex's light samples, or
-//                 sample the next bounce (closest-hit queue) -- on opaque,
-//                 untextured surfaces handing that to
+//                 continue the path: refract (closest-hit queue), or hand a
+//                 reflection to
 //   bounce_kernel the reflection sample and the next closest-hit ray;
 //   nee_kernel    shadow answers of terminating-vertex light samples and the
 //                 workers shade_kernel handed over: emit, then draw the next
@@ -522,35 +522,38 @@ RMN_D int shade_hit(const Job* J, const Pool& P, int w, RmnRng& rng, int4& ph, c
       P.nk[w] = make_int4(0, cnt, sf.entering ? 1 : 0, reflect ? 0 : 1);
       phase = PH_NEE;
     }
-  } else if (!GLASS && !s.has_tex) {
-    // the bounce of an opaque, untextured surface: bounce_kernel samples it
-    // from this record (the NEE vertex's slots, free at a bounce)
+  } else if (!GLASS || reflect) {
+    // a reflection: bounce_kernel samples it from this record (the NEE
+    // vertex's slots and light weights, free at a bounce)
     float4* nv = P.nv + 6 * (size_t)w;
     nv[0] = make_float4(sf.pos.x, sf.pos.y, sf.pos.z, p_rr);
     nv[1] = make_float4(sf.shapeN.x, sf.shapeN.y, sf.shapeN.z, sf.roughness);
     nv[2] = make_float4(sf.surfN.x, sf.surfN.y, sf.surfN.z, sf.metallic);
     nv[3] = make_float4(sf.base.x, sf.base.y, sf.base.z, sf.eta);
     nv[4] = make_float4(V.x, V.y, V.z, sf.specular);
-    nv[5] = make_float4(rf, sf.opacity, nee ? 1.0f : 0.0f, 0.0f);
+    nv[5] = make_float4(rf, sf.opacity, nee ? 1.0f : 0.0f, pr);
+    if (GLASS) P.lw[2 * w] = make_float4(absorb.x, absorb.y, absorb.z, 0.0f);
+    if (s.has_tex) {
+      RayDiff nx;
+      nx.dPdx = hpx;
+      nx.dPdy = hpy;
+      calc_dDdxy(dir, sf.surfN, diff, nx.dDdx, nx.dDdy);
+      store_diff(P, w, nx);
+    }
     phase = PH_BOUNCE;
   } else {
     float3 nd, wv;
     int nf = 0;
-    if (reflect) {
-      sample_reflect(sf, V, rng, nd, wv, nf);
-      wv = wv / pr;
-    } else if (GLASS) {
-      if (fabsf(sf.eta - 1.0f) < RMN_EPS) {  // inside a medium: straight on
-        nd = dir;
-        wv = f3(1.0f);
-      } else {
-        sample_btdf(sf, V, rng, nd, wv, nf);
-        wv = wv * (1.0f - F);
-      }
-      wv = wv / (1.0f - pr);
-      if (sf.entering) med.insert(sf.id, ior, sf.base);
-      else med.erase(sf.id);
+    if (fabsf(sf.eta - 1.0f) < RMN_EPS) {  // inside a medium: straight on
+      nd = dir;
+      wv = f3(1.0f);
+    } else {
+      sample_btdf(sf, V, rng, nd, wv, nf);
+      wv = wv * (1.0f - F);
     }
+    wv = wv / (1.0f - pr);
+    if (sf.entering) med.insert(sf.id, ior, sf.base);
+    else med.erase(sf.id);
     if (nee) wv = wv / p_rr;
     if (any_finite3(nd) && depth != p.maxd) {
       wv = wv * absorb;
@@ -562,14 +565,7 @@ RMN_D int shade_hit(const Job* J, const Pool& P, int w, RmnRng& rng, int4& ph, c
         P.pa[w] = pa;
       }
       P.ro[w] = make_float4(sf.pos.x, sf.pos.y, sf.pos.z, RMN_EPS);
-      P.rd[w] = make_float4(nd.x, nd.y, nd.z, INFINITY);
-      if (s.has_tex && reflect) {  // a refracted ray keeps its differential
-        RayDiff nx;
-        nx.dPdx = hpx;
-        nx.dPdy = hpy;
-        calc_dDdxy(dir, sf.surfN, diff, nx.dDdx, nx.dDdy);
-        store_diff(P, w, nx);
-      }
+      P.rd[w] = make_float4(nd.x, nd.y, nd.z, INFINITY);  // with textures it keeps its differential
       ph.z = depth + 1;
       ph.w = nee ? FL_EXCLUDE : 0;
       phase = PH_WAIT_CLOSEST;
@@ -641,11 +637,11 @@ __global__ void __launch_bounds__(128, 8) shade_kernel(const Job* __restrict__ j
   }
 }
 
-// The bounces shade_kernel handed over (opaque, untextured surfaces): the
-// reflection sample of sampleRay (src/render.cpp:238-250) and the next
-// closest-hit ray, in the operations and order of shade_hit's own bounce
-// (pr = 1 and no absorption on an opaque surface). A warp here runs the
-// reflection sampler alone, not beside emission and light-sample starts.
+// The reflections shade_kernel handed over: the sample of sampleRay
+// (src/render.cpp:238-250), divided by P_reflect and P_RR and absorbed over
+// the segment that led here, and the next closest-hit ray. A warp here runs the
+// reflection sampler alone, not beside emission, refractions and light-sample
+// starts.
 RMN_D int bounce_step(const Job* __restrict__ jobs, const Pool& P, int w) {
   int4 ph, un;
   long long uid;
@@ -667,17 +663,20 @@ RMN_D int bounce_step(const Job* __restrict__ jobs, const Pool& P, int w) {
   sf.specular = e.w;
   sf.opacity = f.y;
   const float3 V = f3(e.x, e.y, e.z);
-  const float p_rr = a.w, rf = f.x;
+  const float p_rr = a.w, rf = f.x, pr = f.w;
   const bool nee = f.z != 0.0f;
   const int depth = ph.z;
   float3 nd, wv;
   int nf = 0;
   sample_reflect(sf, V, rng, nd, wv, nf);
-  wv = wv / 1.0f;  // / P_reflect (1 on an opaque surface)
+  wv = wv / pr;
   if (nee) wv = wv / p_rr;
   int phase = PH_SLOT;
   if (any_finite3(nd) && depth != p.maxd) {
-    wv = wv * f3(1.0f);  // no absorption outside media
+    if (p.glass) {  // absorption over the segment just traced
+      const float4 ab = P.lw[2 * w];
+      wv = wv * f3(ab.x, ab.y, ab.z);
+    }
     const float4 pb = P.pb[w];
     float3 thr = f3(pb.x, pb.y, pb.z) * wv;
     P.pb[w] = make_float4(thr.x, thr.y, thr.z, rf);
