@@ -1647,8 +1647,8 @@ __device__ __forceinline__ unsigned ray_bin(const Job* __restrict__ jobs, const 
   if (root >= 0) {
     const DevNode* n = nodes + root;
     const float4 A = __ldg(&n->a), B = __ldg(&n->b), C = __ldg(&n->c);
-    const float lx = fminf(A.x, B.z), ly = fminf(A.y, B.w), lz = fminf(A.z, C.x);
-    const float hx = fmaxf(A.w, C.y), hy = fmaxf(B.x, C.z), hz = fmaxf(B.y, C.w);
+    const float lx = fminf(A.x, B.x), ly = fminf(A.y, B.y), lz = fminf(C.x, C.z);
+    const float hx = fmaxf(A.z, B.z), hy = fmaxf(A.w, B.w), hz = fmaxf(C.y, C.w);
     auto q = [](float v, float lo, float hi) {
       const float f = (v - lo) / fmaxf(hi - lo, 1e-20f) * 8.0f;
       return (unsigned)fminf(fmaxf(f, 0.0f), 7.0f);

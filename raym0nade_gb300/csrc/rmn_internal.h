@@ -84,10 +84,12 @@ constexpr int kOccSteps = 10;  // occlusion queries with pending leaves (trace.c
 // so one node fetch serves the reference's two rayInBox tests
 // (src/bvh.cpp:74-75). Child reference >= 0: inner node index; < 0: leaf,
 // ~(first_triangle << 4 | count).
+// The bounds lie in the pairs that the box tests' two-wide subtractions and
+// multiplications take.
 struct __align__(16) DevNode {
-  float4 a;  // L.lo.x L.lo.y L.lo.z L.hi.x
-  float4 b;  // L.hi.y L.hi.z R.lo.x R.lo.y
-  float4 c;  // R.lo.z R.hi.x R.hi.y R.hi.z
+  float4 a;  // L.lo.x L.lo.y L.hi.x L.hi.y
+  float4 b;  // R.lo.x R.lo.y R.hi.x R.hi.y
+  float4 c;  // L.lo.z L.hi.z R.lo.z R.hi.z
   int4 d;    // L ref, R ref, -, -
 };
 RMN_HD int leaf_ref(int first, int count) { return ~((first << 4) | count); }

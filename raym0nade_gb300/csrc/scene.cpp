@@ -150,9 +150,9 @@ struct Flattener {
     int r = ref_of(u << 1 | 1, depth + 1);
     const HeapNode &L = heap[u << 1], &R = heap[u << 1 | 1];
     DevNode& d = out[me];
-    d.a = make_float4(L.lo.x, L.lo.y, L.lo.z, L.hi.x);
-    d.b = make_float4(L.hi.y, L.hi.z, R.lo.x, R.lo.y);
-    d.c = make_float4(R.lo.z, R.hi.x, R.hi.y, R.hi.z);
+    d.a = make_float4(L.lo.x, L.lo.y, L.hi.x, L.hi.y);
+    d.b = make_float4(R.lo.x, R.lo.y, R.hi.x, R.hi.y);
+    d.c = make_float4(L.lo.z, L.hi.z, R.lo.z, R.hi.z);
     d.d = make_int4(l, r, 0, 0);
     return me;
   }

@@ -62,6 +62,39 @@ RMN_D bool box_hit(const TRay& r, float3 lo, float3 hi, float tmin, float tmax, 
   return L < R;
 }
 
+// Two floats in one 64-bit register pair: a subtraction or multiplication of
+// the pair is one instruction, each half rounded as the single operation.
+RMN_D unsigned long long pair2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+RMN_D float2 halves(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+// ((a - o.x) * i.x, (b - o.y) * i.y): slab distances.
+RMN_D float2 slab2(float a, float b, unsigned long long o, unsigned long long i) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pair2(a, b)), "l"(o));
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(r), "l"(i));
+  return halves(r);
+}
+
+// box_hit without branches, for rays with no axis under the origin-inside
+// rule (r.par == 0), on a box's six slab distances (lo and hi of x and y, then
+// z). The smaller of an axis's two is its entry (box_hit's choice by the sign
+// of 1/d: multiplication and subtraction round monotonely and lo <= hi).
+// Whether the box is hit is box_hit's answer; tL is box_hit's when it is.
+RMN_D bool box_run(float2 lo, float2 hi, float2 z, float tmin, float tmax, float& tL) {
+  const float L1 = fmaxf(tmin, fminf(lo.x, hi.x)), R1 = fminf(tmax, fmaxf(lo.x, hi.x)) + RMN_EPS;
+  const float L2 = fmaxf(L1, fminf(lo.y, hi.y)), R2 = fminf(R1, fmaxf(lo.y, hi.y)) + RMN_EPS;
+  const float L3 = fmaxf(L2, fminf(z.x, z.y)), R3 = fminf(R2, fmaxf(z.x, z.y)) + RMN_EPS;
+  tL = L3;
+  return !(L1 > R1) && !(L2 > R2) && L3 < R3;
+}
+
 // A box test that accepts every box box_hit accepts (and a few more), for
 // queries whose answer does not depend on the order of visits or on the
 // entry distances (occlusion), on rays with no axis under the
@@ -71,12 +104,9 @@ RMN_D bool box_hit(const TRay& r, float3 lo, float3 hi, float tmin, float tmax, 
 // g(min(g(min(g(min(tmax, fx)), fy)), fz)) with g(m) = RN(m + eps),
 // monotone with g(m) >= m, which is at most g(g(g(min(tmax, fx, fy, fz))))
 // = R here. So box_hit's tL < tR implies L < R.
-RMN_D bool box_any(const TRay& r, float3 lo, float3 hi, float tmin, float tmax, float& tL) {
-  const float x0 = (lo.x - r.o.x) * r.inv.x, x1 = (hi.x - r.o.x) * r.inv.x;
-  const float y0 = (lo.y - r.o.y) * r.inv.y, y1 = (hi.y - r.o.y) * r.inv.y;
-  const float z0 = (lo.z - r.o.z) * r.inv.z, z1 = (hi.z - r.o.z) * r.inv.z;
-  const float L = fmaxf(fmaxf(tmin, fminf(x0, x1)), fmaxf(fminf(y0, y1), fminf(z0, z1)));
-  float R = fminf(fminf(tmax, fmaxf(x0, x1)), fminf(fmaxf(y0, y1), fmaxf(z0, z1)));
+RMN_D bool box_any(float2 lo, float2 hi, float2 z, float tmin, float tmax, float& tL) {
+  const float L = fmaxf(fmaxf(tmin, fminf(lo.x, hi.x)), fmaxf(fminf(lo.y, hi.y), fminf(z.x, z.y)));
+  float R = fminf(fminf(tmax, fmaxf(lo.x, hi.x)), fminf(fmaxf(lo.y, hi.y), fmaxf(z.x, z.y)));
   R += RMN_EPS;
   R += RMN_EPS;
   R += RMN_EPS;
@@ -191,12 +221,27 @@ RMN_D int inner_step(const DevNode* __restrict__ nodes, const TRay& r, float tmi
   if (COUNT) cnt->inner++;
   float tl0, tl1;
   bool h0, h1;
-  if (WIDE && r.par == 0) {
-    h0 = box_any(r, f3(A.x, A.y, A.z), f3(A.w, B.x, B.y), tmin, tmax, tl0);
-    h1 = box_any(r, f3(B.z, B.w, C.x), f3(C.y, C.z, C.w), tmin, tmax, tl1);
-  } else {
-    h0 = box_hit(r, f3(A.x, A.y, A.z), f3(A.w, B.x, B.y), tmin, tmax, tl0);
-    h1 = box_hit(r, f3(B.z, B.w, C.x), f3(C.y, C.z, C.w), tmin, tmax, tl1);
+  bool fast = r.par == 0;
+  if (fast) {
+    const unsigned long long oxy = pair2(r.o.x, r.o.y), ixy = pair2(r.inv.x, r.inv.y);
+    const unsigned long long oz = pair2(r.o.z, r.o.z), iz = pair2(r.inv.z, r.inv.z);
+    const float2 la = slab2(A.x, A.y, oxy, ixy), lb = slab2(A.z, A.w, oxy, ixy), lz = slab2(C.x, C.y, oz, iz);
+    const float2 ra = slab2(B.x, B.y, oxy, ixy), rb = slab2(B.z, B.w, oxy, ixy), rz = slab2(C.z, C.w, oz, iz);
+    if (WIDE) {
+      h0 = box_any(la, lb, lz, tmin, tmax, tl0);
+      h1 = box_any(ra, rb, rz, tmin, tmax, tl1);
+    } else {
+      h0 = box_run(la, lb, lz, tmin, tmax, tl0);
+      h1 = box_run(ra, rb, rz, tmin, tmax, tl1);
+      // only one box hit, and entered within the added eps of tmax: whether it
+      // is taken depends on which child counts as the nearer, so on the other
+      // box's distance where box_hit stopped
+      fast = h0 == h1 || (h0 ? tl0 : tl1) < tmax;
+    }
+  }
+  if (!fast) {
+    h0 = box_hit(r, f3(A.x, A.y, C.x), f3(A.z, A.w, C.y), tmin, tmax, tl0);
+    h1 = box_hit(r, f3(B.x, B.y, C.z), f3(B.z, B.w, C.w), tmin, tmax, tl1);
   }
   int nref, fref;
   bool hn, hf;
