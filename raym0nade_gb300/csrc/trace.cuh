@@ -366,8 +366,7 @@ RMN_D int coop_nodes(const DevNode* __restrict__ nodes, const TRay& r, float tmi
   for (int step = 0; step < steps; ++step) {
     const bool g = go && res == 0 && t.ti >= t.te;
     if (!__any_sync(0xffffffffu, g)) break;
-    if (!g) continue;
-    if (t.pop) {
+    if (g && t.pop) {
       t.pop = false;
       for (;;) {
         if (t.sp == 0) {
@@ -381,20 +380,14 @@ RMN_D int coop_nodes(const DevNode* __restrict__ nodes, const TRay& r, float tmi
           break;
         }
       }
-      if (res) continue;
     }
-    if (t.cur >= 0) {
+    const bool live = g && res == 0;
+    if (live && t.cur >= 0) {
       const int k = inner_step<COUNT>(nodes, r, tmin, t.tmax, t.cur, t.sp, t.stack, cnt);
-      if (k == -2) {
-        res = -2;
-        continue;
-      }
-      if (k == 1) {
-        t.pop = true;
-        continue;
-      }
+      if (k == -2) res = -2;
+      t.pop = k == 1;
     }
-    if (t.cur < 0) {  // a leaf: its triangles wait for phase 2, then a pop
+    if (live && t.cur < 0 && res == 0 && !t.pop) {  // a leaf: its triangles wait for phase 2, then a pop
       const int x = ~t.cur;
       const int count = x & 15;
       if (COUNT) { cnt->leaves++; cnt->tris += count; }
@@ -532,8 +525,7 @@ RMN_D int occ_nodes(const DevNode* __restrict__ nodes, const TRay& r, float tmin
   for (int step = 0; step < steps; ++step) {
     const bool g = go && res == 0 && t.c1 == 0;
     if (!__any_sync(0xffffffffu, g)) break;
-    if (!g) continue;
-    if (t.pop) {
+    if (g && t.pop) {
       t.pop = false;
       for (;;) {
         if (t.sp == 0) {
@@ -547,20 +539,14 @@ RMN_D int occ_nodes(const DevNode* __restrict__ nodes, const TRay& r, float tmin
           break;
         }
       }
-      if (res) continue;
     }
-    if (t.cur >= 0) {
+    const bool live = g && res == 0;
+    if (live && t.cur >= 0) {
       const int k = inner_step<COUNT, true>(nodes, r, tmin, tmax, t.cur, t.sp, t.stack, cnt);
-      if (k == -2) {
-        res = -2;
-        continue;
-      }
-      if (k == 1) {
-        t.pop = true;
-        continue;
-      }
+      if (k == -2) res = -2;
+      t.pop = k == 1;
     }
-    if (t.cur < 0) {  // a leaf: kept pending, and on to the next node
+    if (live && t.cur < 0 && res == 0 && !t.pop) {  // a leaf: kept pending, and on to the next node
       const int x = ~t.cur;
       const int count = x & 15;
       if (COUNT) { cnt->leaves++; cnt->tris += count; }
