@@ -70,28 +70,24 @@ void release(Arg& a, cudaStream_t st) {
   a.owned = false;
 }
 
-// Device status word of one call.
+// Status word of one call: kernels on the call's stream write it.
 struct Status {
-  int* dev = nullptr;
-  rmn_status init(cudaStream_t st) {
-    cudaError_t e = rmn::staging_malloc(reinterpret_cast<void**>(&dev), sizeof(int), st);
-    if (e != cudaSuccess) return cuda_fail(e, "staging allocation (status)");
-    e = cudaMemsetAsync(dev, 0, sizeof(int), st);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync (status)");
+  int* word = nullptr;
+  rmn_status init() {
+    cudaError_t e = rmn::acquire_status(&word);
+    if (e != cudaSuccess) return cuda_fail(e, "pinned allocation (status)");
     return RMN_OK;
   }
-  rmn_status check(cudaStream_t st, const char* what) {
-    int h = 0;
-    cudaError_t e = cudaMemcpyAsync(&h, dev, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_fail(e, what);
+  // after the stream's synchronisation
+  rmn_status check(const char* what) const {
+    const int h = *reinterpret_cast<volatile int*>(word);
     if (h == kDevStackOverflow) return fail(RMN_ERR_DEVICE_LIMIT, "%s: traversal stack bound reached", what);
     if (h != kDevOk) return fail(RMN_ERR_DEVICE_LIMIT, "%s: device status %d", what, h);
     return RMN_OK;
   }
-  void free(cudaStream_t st) {
-    if (dev) cudaFreeAsync(dev, st);
-    dev = nullptr;
+  void free() {
+    rmn::release_status(word);
+    word = nullptr;
   }
 };
 }  // namespace
@@ -359,22 +355,21 @@ static rmn_status trace_common(rmn_scene* scene, const rmn_ray* rays, int64_t n,
   Status status;
   rmn_status r = stage_in(rays, (size_t)n * sizeof(rmn_ray), st, &in);
   if (r == RMN_OK) r = stage_out(out, out_bytes, st, &o);
-  if (r == RMN_OK) r = status.init(st);
+  if (r == RMN_OK) r = status.init();
   if (r == RMN_OK) {
     cudaError_t e = shadow ? launch_trace_shadow(scene->dev, static_cast<const rmn_ray*>(in.dev), n,
-                                                 static_cast<uint8_t*>(o.dev), status.dev, st)
+                                                 static_cast<uint8_t*>(o.dev), status.word, st)
                            : launch_trace_closest(scene->dev, static_cast<const rmn_ray*>(in.dev), n,
-                                                  static_cast<rmn_hit*>(o.dev), status.dev, st);
+                                                  static_cast<rmn_hit*>(o.dev), status.word, st);
     if (e != cudaSuccess) r = cuda_fail(e, shadow ? "trace_shadow launch" : "trace_closest launch");
   }
   if (r == RMN_OK) r = finish_out(out, out_bytes, st, o);
-  rmn_status r2 = status.dev ? status.check(st, shadow ? "rmn_trace_shadow" : "rmn_trace_closest") : RMN_OK;
   release(in, st);
   release(o, st);
-  status.free(st);
   cudaError_t e = cudaStreamSynchronize(st);
-  if (r == RMN_OK) r = r2;
   if (r == RMN_OK && e != cudaSuccess) r = cuda_fail(e, "stream synchronize");
+  if (r == RMN_OK) r = status.check(shadow ? "rmn_trace_shadow" : "rmn_trace_closest");
+  status.free();
   return r;
 }
 
@@ -628,7 +623,7 @@ static rmn_status render_one(rmn_scene* scene, const rmn_render_args* args, cons
   if (r == RMN_OK && b) r = batch_status(b, st);
   for (Arg* x : {&dd, &ds, &id, &is, &gb, &dr}) release(*x, st);
   cudaError_t e = cudaStreamSynchronize(st);
-  batch_destroy(b);
+  batch_destroy(b, r == RMN_OK && e == cudaSuccess);
   if (r == RMN_OK && e != cudaSuccess) r = cuda_fail(e, "stream synchronize");
   return r;
 }
@@ -880,7 +875,7 @@ rmn_status rmn_batch_autotune(const rmn_batch_item* items, int32_t n, float pixe
     if (r == RMN_OK) r = batch_status(b, st);
     float ms = 0.0f;
     if (r == RMN_OK && cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) r = fail(RMN_ERR_CUDA, "event timing");
-    batch_destroy(b);
+    batch_destroy(b, false);
     if (r != RMN_OK) break;
     best.candidates++;
     if (is_default) best.default_ms = ms;
@@ -938,7 +933,7 @@ rmn_status rmn_batch_profile(rmn_batch* batch, rmn_render_profile* out, void* st
 rmn_status rmn_batch_destroy(rmn_batch* batch) {
   clear_error();
   if (!batch) return RMN_OK;
-  batch_destroy(batch->state);
+  batch_destroy(batch->state, false);
   delete batch;
   return RMN_OK;
 }

@@ -17,6 +17,8 @@
 #include <map>
 #include <mutex>
 #include <unordered_map>
+#include <utility>
+#include <vector>
 
 #include "rmn_host.h"
 
@@ -57,6 +59,17 @@ cudaError_t staging_pool(cudaMemPool_t* out) {
   *out = pool;
   return cudaSuccess;
 }
+
+// Status words, 64 bytes apart in pinned pages of 64: at most as many as calls
+// were ever in flight at once, rounded up to a page.
+constexpr int kStatusStride = 16;
+std::mutex g_status_mu;
+std::vector<int*> g_status_free;
+std::vector<int*> g_status_pages;
+
+// Launch limits by device and kernel: they do not change.
+std::mutex g_limit_mu;
+std::map<std::pair<int, std::pair<const void*, int>>, int> g_limits;
 
 struct DeviceCache {
   std::multimap<size_t, void*> free_blocks;  // size -> block
@@ -125,7 +138,54 @@ cudaError_t staging_malloc(void** p, size_t bytes, cudaStream_t st) {
   return cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, st);
 }
 
+cudaError_t acquire_status(int** word) {
+  std::lock_guard<std::mutex> lock(g_status_mu);
+  if (g_status_free.empty()) {
+    int* page = nullptr;
+    cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&page), 64 * kStatusStride * sizeof(int),
+                                  cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e != cudaSuccess) return e;
+    g_status_pages.push_back(page);
+    for (int i = 0; i < 64; ++i) g_status_free.push_back(page + i * kStatusStride);
+  }
+  *word = g_status_free.back();
+  g_status_free.pop_back();
+  **word = 0;
+  return cudaSuccess;
+}
+
+void release_status(int* word) {
+  if (!word) return;
+  std::lock_guard<std::mutex> lock(g_status_mu);
+  g_status_free.push_back(word);
+}
+
+int device_sms() {
+  return blocks_per_sm(nullptr, 0);
+}
+
+int blocks_per_sm(const void* kernel, int threads) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(g_limit_mu);
+  int& v = g_limits[{dev, {kernel, threads}}];
+  if (v <= 0) {
+    if (kernel) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kernel, threads, 0);
+    else cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    if (v < 1) v = 1;
+  }
+  return v;
+}
+
 void release_cached_memory() {
+  {
+    std::lock_guard<std::mutex> lock(g_status_mu);
+    if (g_status_free.size() == 64 * g_status_pages.size()) {  // no call in flight
+      for (int* p : g_status_pages) cudaFreeHost(p);
+      g_status_pages.clear();
+      g_status_free.clear();
+    }
+  }
   {
     std::lock_guard<std::mutex> lock(g_pool_mu);
     for (auto& kv : g_pools) cudaMemPoolTrimTo(kv.second, 0);

@@ -1770,18 +1770,10 @@ __global__ void __launch_bounds__(128) finalize_kernel(const Job* __restrict__ j
   if (J.dropped) J.dropped[pixel] = dropped;
 }
 
-int device_sms() {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
+using rmn::device_sms;
 template <class K>
 int blocks_per_sm(K kernel) {
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0);
-  return per_sm < 1 ? 1 : per_sm;
+  return rmn::blocks_per_sm((const void*)kernel, 128);
 }
 
 }  // namespace
@@ -1809,7 +1801,7 @@ struct BatchState {
   JobTable table;
   Job* d_jobs = nullptr;
   CtlBlock* d_ctl = nullptr;
-  int* d_status = nullptr;
+  int* d_status = nullptr;    // pinned status word (acquire_status)
   float4* d_parts = nullptr;
   int lanes = 1;
   bool alpha = false;         // some job's scene has alpha-tested materials
@@ -2017,7 +2009,7 @@ static cudaError_t launch_block(BatchState* b, int lane, long long n, cudaStream
 
 // The last workers of every lane (n[l] of lane l), the lanes side by side.
 static cudaError_t launch_blocks(BatchState* b, const long long* n, cudaStream_t st) {
-  cudaError_t e = cudaEventRecord(b->fork, st);
+  cudaError_t e = b->lanes > 1 ? cudaEventRecord(b->fork, st) : cudaSuccess;
   for (int l = 0; l < b->lanes && e == cudaSuccess; ++l) {
     if (n[l] <= 0) continue;
     cudaStream_t ls = l == 0 ? st : b->ls[l];
@@ -2165,7 +2157,7 @@ static rmn_status run(BatchState* b, cudaStream_t st, Counters* ctr, cudaEvent_t
   return RMN_OK;
 }
 
-void batch_destroy(BatchState* b) {
+void batch_destroy(BatchState* b, bool idle) {
   if (!b) return;
   if (b->init_exec) cudaGraphExecDestroy(b->init_exec);
   if (b->chunk_exec) cudaGraphExecDestroy(b->chunk_exec);
@@ -2178,7 +2170,8 @@ void batch_destroy(BatchState* b) {
   if (b->upd) cudaEventDestroy(b->upd);
   // the blocks go back to the cache for the next batch: no work of this
   // batch may still run on them (cudaFree would have waited likewise)
-  cudaDeviceSynchronize();
+  if (!idle) cudaDeviceSynchronize();
+  release_status(b->d_status);
   if (b->h_jobs) cudaFreeHost(b->h_jobs);
   for (void* p : b->allocs) cached_free(p);
   delete b;
@@ -2266,10 +2259,15 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
   b->use_graph = use_graph;
   b->binned = ray_order != 0;
   b->lanes = lanes > 0 ? std::min(lanes, kMaxLanes) : default_lanes(b->table.total_units);
-  // workers per lane; no more lanes and workers than there are units; the
-  // default pool halves while the workers would take more than a quarter of
-  // the free device memory
+  // workers per lane; no more lanes and workers than there are units, nor, for a
+  // render without wavefront, than are resident; the default pool halves while
+  // the workers would take more than a quarter of the free device memory
   long long per = pool_workers > 0 ? pool_workers : kDefaultPoolWorkers;
+  b->direct = b->table.total_units <= kDirectUnits;
+  if (b->direct) {
+    b->lanes = 1;
+    per = std::min(per, std::min(block_capacity(), b->table.total_units));
+  }
   if (pool_workers <= 0) {
     bool glass = false, tex = false;
     for (const Job& j : b->table.jobs) {
@@ -2278,11 +2276,6 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
     }
     const size_t budget = free_device_bytes() / 4;
     while (per > 4096 && worker_bytes(glass, tex) * (size_t)per * b->lanes > budget) per /= 2;
-  }
-  b->direct = b->table.total_units <= kDirectUnits;
-  if (b->direct) {
-    b->lanes = 1;
-    per = std::min(per, block_capacity());
   }
   while (b->lanes > 1 && (long long)b->lanes * 128 > b->table.total_units) --b->lanes;
   per = std::min<long long>(per, (b->table.total_units + b->lanes - 1) / b->lanes);
@@ -2298,7 +2291,6 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
   const size_t jb = sizeof(Job) * b->table.jobs.size();
   alloc((void**)&b->d_jobs, jb);
   alloc((void**)&b->d_ctl, sizeof(CtlBlock));
-  alloc((void**)&b->d_status, sizeof(int));
   alloc((void**)&b->d_parts, sizeof(float4) * RMN_PART_F4 * (size_t)b->table.total_units);
   Pool P{};
   P.W = (int)W;
@@ -2375,12 +2367,14 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
     }
   }
   if (e == cudaSuccess) e = cudaMemcpy(b->d_jobs, b->table.jobs.data(), jb, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(b->d_status, 0, sizeof(int));
-  for (int l = 0; l < b->lanes && e == cudaSuccess; ++l) {
+  if (e == cudaSuccess) e = acquire_status(&b->d_status);
+  // streams and events for the lanes beside the caller's stream, and one to
+  // capture graphs on
+  for (int l = use_graph ? 0 : 1; l < b->lanes && e == cudaSuccess; ++l) {
     e = cudaStreamCreateWithFlags(&b->ls[l], cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[l], cudaEventDisableTiming);
+    if (e == cudaSuccess && l > 0) e = cudaEventCreateWithFlags(&b->join[l], cudaEventDisableTiming);
   }
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+  if (e == cudaSuccess && b->lanes > 1) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
   if (e == cudaSuccess && use_graph) {
     // One chunk graph: the lanes' iterations as parallel branches (fork and
     // join through events between the lane streams), so their kernels overlap.
@@ -2390,7 +2384,7 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
     if (e == cudaSuccess) e = capture(c0, [&] { return launch_finalize(b, c0); }, &b->fin_exec);
   }
   if (e != cudaSuccess) {
-    batch_destroy(b);
+    batch_destroy(b, false);
     return cuda_fail(e, "batch setup");
   }
   (void)st;
@@ -2473,10 +2467,9 @@ size_t batch_device_bytes(const RenderItem* items_in, int n, int pool_workers, i
 int batch_items(const BatchState* b) { return (int)b->table.jobs.size(); }
 
 rmn_status batch_status(BatchState* b, cudaStream_t st) {
-  int h = 0;
-  cudaError_t e = cudaMemcpyAsync(&h, b->d_status, sizeof(int), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  const cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(e, "render");
+  const int h = *reinterpret_cast<volatile int*>(b->d_status);
   if (h == kDevMediaOverflow) return fail(RMN_ERR_DEVICE_LIMIT, "render: a path entered more than %d nested media",
                                           RMN_MEDIA - 1);
   if (h) return fail(RMN_ERR_DEVICE_LIMIT, "render: traversal stack bound reached");

@@ -143,6 +143,15 @@ void release_cached_memory();
 // A stream-ordered allocation from the library's staging pool (devmem.cpp),
 // freed with cudaFreeAsync.
 cudaError_t staging_malloc(void** p, size_t bytes, cudaStream_t st);
+// A status word of one call: pinned host memory that kernels write and the host
+// reads once the call's stream is synchronised (no device word to clear, no
+// copy back). acquire gives it zeroed; the words are kept for later calls.
+cudaError_t acquire_status(int** word);
+void release_status(int* word);
+// SMs of the current device, and the blocks of `threads` threads (no dynamic
+// shared memory) an SM of it holds of a kernel: asked of the runtime once.
+int device_sms();
+int blocks_per_sm(const void* kernel, int threads);
 // Forgets the device addresses rmn_compose_noalloc resolved (after a device
 // reset they name nothing); the next call on each device resolves them anew.
 void noalloc_forget_addresses();
@@ -167,7 +176,8 @@ void default_slots_per_unit(const RenderItem* items, int n, int* S);
 int batch_items(const BatchState* b);
 rmn_status batch_status(BatchState* b, cudaStream_t st);
 rmn_status batch_profile(BatchState* b, cudaStream_t st, RenderProfileData* prof);
-void batch_destroy(BatchState* b);
+// idle: no work of the batch is left on the device (its stream is synchronised).
+void batch_destroy(BatchState* b, bool idle);
 
 // Adjoint of one render (adjoint.cu): device buffers only; dmat receives
 // num_materials * RMN_GRAD_PER_MATERIAL floats.

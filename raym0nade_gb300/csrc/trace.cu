@@ -28,6 +28,9 @@ __global__ void __launch_bounds__(128, RMN_COOP_BLOCKS(STACK)) trace_kernel(DevS
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   bool active = false, retired = lane >= use;
+  // without a counter: each warp its own `use` rays
+  const unsigned long long first = (unsigned long long)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * use;
+  bool fetched = false;
   int64_t i = 0;
   TRay r;
   float tmin = 0.0f, aim = 0.0f, restart = 0.0f;
@@ -47,7 +50,9 @@ __global__ void __launch_bounds__(128, RMN_COOP_BLOCKS(STACK)) trace_kernel(DevS
     if (need) {
       const int leader = __ffs(need) - 1;
       unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(need));
+      if (!next) base = fetched ? (unsigned long long)n : first;
+      else if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(need));
+      fetched = true;
       base = __shfl_sync(0xffffffffu, base, leader);
       if (!active && !retired) {
         i = (int64_t)(base + __popc(need & lt));
@@ -103,6 +108,9 @@ __global__ void __launch_bounds__(128, RMN_OCC_BLOCKS) occ_kernel(DevScene s, co
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   bool active = false, retired = lane >= use;
+  // without a counter: each warp its own `use` rays
+  const unsigned long long first = (unsigned long long)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * use;
+  bool fetched = false;
   int64_t i = 0;
   TRay r;
   float aim = 0.0f;
@@ -116,7 +124,9 @@ __global__ void __launch_bounds__(128, RMN_OCC_BLOCKS) occ_kernel(DevScene s, co
     if (need) {
       const int leader = __ffs(need) - 1;
       unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(need));
+      if (!next) base = fetched ? (unsigned long long)n : first;
+      else if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(need));
+      fetched = true;
       base = __shfl_sync(0xffffffffu, base, leader);
       if (!active && !retired) {
         i = (int64_t)(base + __popc(need & lt));
@@ -142,22 +152,13 @@ __global__ void __launch_bounds__(128, RMN_OCC_BLOCKS) occ_kernel(DevScene s, co
   }
 }
 
-int persistent_blocks(const void* kernel, int threads) {
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
-  if (per_sm < 1) per_sm = 1;
-  return sms * per_sm;
-}
-
 template <bool SHADOW, int STACK>
-void launch_kernel(const DevScene& s, const float4* rays, int64_t n, float4* hits, uint8_t* occ,
-                   unsigned long long* next, int* status, cudaStream_t stream) {
+cudaError_t launch_kernel(const DevScene& s, const float4* rays, int64_t n, float4* hits, uint8_t* occ, int* status,
+                          cudaStream_t stream) {
   const int threads = 128;
   const bool order_free = SHADOW && !s.has_alpha;
-  int blocks = order_free ? persistent_blocks((const void*)occ_kernel<STACK>, threads)
-                          : persistent_blocks((const void*)trace_kernel<SHADOW, STACK>, threads);
+  const void* kernel = order_free ? (const void*)occ_kernel<STACK> : (const void*)trace_kernel<SHADOW, STACK>;
+  int blocks = rmn::device_sms() * rmn::blocks_per_sm(kernel, threads);
   // the rays go over all the warps the device holds, `use` of a warp's lanes
   // taking one each: a warp's time is its rays' divergent steps one after the
   // other. With 32 rays a warp while most of the device is idle, 1000 rays of the
@@ -167,33 +168,38 @@ void launch_kernel(const DevScene& s, const float4* rays, int64_t n, float4* hit
   const int64_t warps = (int64_t)blocks * (threads / 32);
   const int use = (int)std::min<int64_t>(32, (n + warps - 1) / warps);
   const int64_t need = (n + (int64_t)use * (threads / 32) - 1) / ((int64_t)use * (threads / 32));
-  if (need < blocks) blocks = (int)need;
-  if (order_free) occ_kernel<STACK><<<blocks, threads, 0, stream>>>(s, rays, n, occ, next, status, use);
-  else trace_kernel<SHADOW, STACK><<<blocks, threads, 0, stream>>>(s, rays, n, hits, occ, next, status, use);
-}
-
-cudaError_t launch(bool shadow, const DevScene& s, const rmn_ray* rays, int64_t n, rmn_hit* hits, uint8_t* occ,
-                   int* status, cudaStream_t stream) {
-  if (n <= 0) return cudaSuccess;
+  if (need <= blocks) {
+    // every ray has its lane: no counter to hand them out
+    blocks = (int)need;
+    if (order_free) occ_kernel<STACK><<<blocks, threads, 0, stream>>>(s, rays, n, occ, nullptr, status, use);
+    else trace_kernel<SHADOW, STACK><<<blocks, threads, 0, stream>>>(s, rays, n, hits, occ, nullptr, status, use);
+    return cudaGetLastError();
+  }
   unsigned long long* next = nullptr;
   cudaError_t e = rmn::staging_malloc(reinterpret_cast<void**>(&next), sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(next, 0, sizeof(unsigned long long), stream);
   if (e == cudaSuccess) {
-    const float4* r = reinterpret_cast<const float4*>(rays);
-    float4* h = reinterpret_cast<float4*>(hits);
-    const bool shallow = s.depth + 1 <= RMN_STACK_SMALL;
-    if (shadow) {
-      if (shallow) launch_kernel<true, RMN_STACK_SMALL>(s, r, n, nullptr, occ, next, status, stream);
-      else launch_kernel<true, RMN_STACK>(s, r, n, nullptr, occ, next, status, stream);
-    } else {
-      if (shallow) launch_kernel<false, RMN_STACK_SMALL>(s, r, n, h, nullptr, next, status, stream);
-      else launch_kernel<false, RMN_STACK>(s, r, n, h, nullptr, next, status, stream);
-    }
+    if (order_free) occ_kernel<STACK><<<blocks, threads, 0, stream>>>(s, rays, n, occ, next, status, use);
+    else trace_kernel<SHADOW, STACK><<<blocks, threads, 0, stream>>>(s, rays, n, hits, occ, next, status, use);
     e = cudaGetLastError();
   }
-  cudaError_t f = cudaFreeAsync(next, stream);
+  const cudaError_t f = cudaFreeAsync(next, stream);
   return e != cudaSuccess ? e : f;
+}
+
+cudaError_t launch(bool shadow, const DevScene& s, const rmn_ray* rays, int64_t n, rmn_hit* hits, uint8_t* occ,
+                   int* status, cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  const float4* r = reinterpret_cast<const float4*>(rays);
+  float4* h = reinterpret_cast<float4*>(hits);
+  const bool shallow = s.depth + 1 <= RMN_STACK_SMALL;
+  if (shadow) {
+    if (shallow) return launch_kernel<true, RMN_STACK_SMALL>(s, r, n, nullptr, occ, status, stream);
+    return launch_kernel<true, RMN_STACK>(s, r, n, nullptr, occ, status, stream);
+  }
+  if (shallow) return launch_kernel<false, RMN_STACK_SMALL>(s, r, n, h, nullptr, status, stream);
+  return launch_kernel<false, RMN_STACK>(s, r, n, h, nullptr, status, stream);
 }
 
 }  // namespace
