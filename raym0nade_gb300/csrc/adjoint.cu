@@ -233,157 +233,115 @@ __device__ __forceinline__ float3 dimg_at(const AdjJob& J, int pixel) {
   return f3(J.dimg[3 * (size_t)pixel], J.dimg[3 * (size_t)pixel + 1], J.dimg[3 * (size_t)pixel + 2]);
 }
 
-// Both kernels: dynamic shared memory holds the block's gradient table (when
-// it fits), flushed to the double-precision sums at the end.
-__device__ __forceinline__ GradSink grad_begin(float* sg, double* gout, int nmats) {
+// The replay: two 256-thread blocks per SM. A lane replays one slot at a time
+// -- a first-vertex light sample or an indirect path -- and takes the next when
+// it is done (slot-major, paths first, from one counter, once kRefill lanes of
+// the warp are free), so no warp waits for its longest path. A round takes every
+// path over one vertex and every light sample, of a first vertex or of one where
+// a path ends, over one shadow ray: bounces, light samples, closest hits, shadow
+// rays, the shading of the hits, the samples' gradients, finished paths. Lanes
+// at different depths thus share every call, and a warp's rays are traced
+// together (coop_nodes / coop_leaves, occ_nodes / occ_leaves).
+//
+// A block's warps go through these phases together: the code of a round is far
+// larger than an SM's instruction caches, and warps in different phases each wait
+// for their own instructions (with every warp going its own way 20 of the 25
+// cycles between two issues, and 6.9 ms for the paths alone; 2.9 in step).
+// 128 registers a thread. 256x256, 32 spp, 16 materials: one block of 512 threads
+// 3.20 ms, two of 256 3.02, four of 128 3.44; one thread per slot, without refill or
+// cooperation, 6.40. 64x64, 8 spp: 0.61, 0.55, 0.57 and 0.58.
+constexpr int kPathThreads = 256;
+constexpr int kPathBlocks = 2;  // per SM
+constexpr int kRefill = 4;
+// From this many lanes a warp on the phases are in step; with fewer the warps'
+// instructions fit side by side and a barrier only makes the short wait for the
+// long (24x24, 4 spp: 202 us without barriers, 230 with).
+constexpr int kInStep = 4;
+enum AdjMode { AM_IDLE = 0, AM_BOUNCE, AM_SAMPLE, AM_FIRST };
+
+// total: all slots of all pixels; use: lanes of a warp that take slots, fewer
+// than 32 where there are not enough slots for every lane of the device.
+__global__ void __launch_bounds__(kPathThreads, kPathBlocks)
+    adjoint_kernel(AdjJob J, long long total, int use, int nmats, double* gout, unsigned long long* next,
+                   int* status) {
+  extern __shared__ __align__(16) unsigned char adj_shared[];
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  AdjTrav& sh = reinterpret_cast<AdjTrav*>(adj_shared)[threadIdx.x >> 5];
+  // the block's gradient table, where it fits, flushed to the double-precision
+  // sums at the end
+  float* sg = reinterpret_cast<float*>(adj_shared + sizeof(AdjTrav) * (kPathThreads / 32));
   const bool use_sh = nmats <= kSharedMats;
   if (use_sh)
-    for (int i = threadIdx.x; i < nmats * kGradPerMat; i += blockDim.x) sg[i] = 0.0f;
+    for (int i = threadIdx.x; i < nmats * kGradPerMat; i += kPathThreads) sg[i] = 0.0f;
   __syncthreads();
-  return GradSink{sg, gout, use_sh};
-}
-__device__ __forceinline__ void grad_end(const GradSink& G, int nmats) {
-  __syncthreads();
-  if (!G.use_sh) return;
-  for (int i = threadIdx.x; i < nmats * kGradPerMat; i += blockDim.x)
-    if (G.sh[i] != 0.0f) atomicAdd(G.gl + i, (double)G.sh[i]);
-}
-
-// Both kernels run in one block per SM whose warps go through the phases of a
-// round together (barriers between them): the code of a round is far larger
-// than an SM's instruction caches, so warps in different phases each wait for
-// their own instructions (20 cycles of 25 a warp waited between two issues
-// while every warp went its own way: 6.9 ms a pass over the paths below;
-// 2.9 ms with the phases in step).
-constexpr int kPathThreads = 512;
-
-// The light-sample slots of the first vertices, slot-major: a warp replays one
-// slot of 32 neighbouring pixels.
-__global__ void __launch_bounds__(kPathThreads, 1)
-    adjoint_light_kernel(AdjJob J, long long total, int nmats, double* gout, int* status) {
-  extern __shared__ __align__(16) unsigned char path_shared[];
-  AdjTrav& sh = reinterpret_cast<AdjTrav*>(path_shared)[threadIdx.x >> 5];
-  GradSink G = grad_begin(reinterpret_cast<float*>(path_shared + sizeof(AdjTrav) * (kPathThreads / 32)), gout, nmats);
+  GradSink G{sg, gout, use_sh};
   const Params& p = J.p;
   const DevScene& s = J.s;
   const long long npx = (long long)p.W * p.H;
-  for (long long t0 = (long long)blockIdx.x * kPathThreads; t0 < total; t0 += (long long)gridDim.x * kPathThreads) {
-    const long long t = t0 + threadIdx.x;
-    const int pixel = (int)(t % npx), j = (int)(t / npx);
-    const float* gb = gbuf_at(J, pixel);
-    bool go = t < total && any_finite3(f3(gb[6], gb[7], gb[8]));  // else a miss: sky only, no material
-    Surf g;
-    float3 Vd, dir;
-    float aim = 0.0f;
-    LSample ls;
-    int li = -1;
-    if (go) {
-      g = first_vertex(J, gb);
-      if (j == 0) G.add(g.id, 4, p.exposure * dot3(dimg_at(J, pixel), g.emis));  // Photo::shade's emission * exposure
-      go = !(len3(g.emis) > 0.0f);
-    }
-    if (go) {
-      RmnRng rng = rmn_rng(p.seed, (uint32_t)pixel, (uint32_t)j);
-      Vd = -norm3(g.pos - p.pos);
-      float lwt[8];
-      float tot = 0.0f;
-      go = (s.sky_w != 0 || light_weights(s, g, Vd, lwt, tot)) &&
-           light_gen(s, g, Vd, lwt, tot, p.spp_d, rng, dir, aim, ls, &li);
-    }
-    __syncthreads();
-    const bool occ = occluded(s, g.pos, dir, aim, go, sh, status);
-    __syncthreads();
-    if (occ || !go) continue;
-    DemodAdj d = demod_adj(g.base, f3(gb[0], gb[1], gb[2]), ls.bsdf, ls.light, ls.weight, dimg_at(J, pixel),
-                           p.exposure);
-    if (!finite1(d.S) || d.S == 0.0f) continue;
-    float3 l, q, lr;
-    brdf_logd(g, Vd, dir, 2, l, q, lr);
-    const float3 A = d.df * ls.bsdf;
-    G.add_base(g.id, A * l - d.S * q + d.dbase);
-    G.add(g.id, 3, dot3(A, lr));
-    if (li >= 0) G.add(__ldg(&s.lights[li].material), 4, d.S);
-  }
-  grad_end(G, nmats);
-}
-
-// The indirect paths. A lane replays one path at a time and takes the next
-// slot when it is done (slot-major, from one counter, once kRefill lanes of
-// the warp are free), so a warp does not wait for its longest path; each round
-// takes every lane's path over one vertex -- the bounce from the vertex it
-// stands at, first or later, the closest hit, its shading, and where the path
-// ends there its light samples -- so that lanes at different depths share every
-// call. The rays of a warp are traced together (coop_nodes / coop_leaves,
-// occ_nodes / occ_leaves).
-//
-// 512 threads of 128 registers: 256, 384, 768 and 1024 threads took 4.85, 4.13,
-// 4.01 and 4.48 ms a call where 512 took 3.88 (256x256, 32 spp, 16 materials;
-// the replay of one path per thread, without refill or cooperation, 6.40).
-constexpr int kRefill = 8;
-
-__global__ void __launch_bounds__(kPathThreads, 1)
-    adjoint_path_kernel(AdjJob J, long long total, int nmats, double* gout, unsigned long long* next, int* status) {
-  extern __shared__ __align__(16) unsigned char path_shared[];
-  const unsigned FULL = 0xffffffffu;
-  AdjTrav& sh = reinterpret_cast<AdjTrav*>(path_shared)[threadIdx.x >> 5];
-  float* sg = reinterpret_cast<float*>(path_shared + sizeof(AdjTrav) * (kPathThreads / 32));
-  const int lane = threadIdx.x & 31;
-  GradSink G = grad_begin(sg, gout, nmats);
-  const Params& p = J.p;
-  const DevScene& s = J.s;
-  const long long npx = (long long)p.W * p.H;
-  bool active = false, more = true;  // more: slots may be left (the same in every lane)
-  // the lane's path: rec[0] is its first vertex, rec[i] its i-th bounce
-  int pixel = 0, j = 0, depth = 0, rfm = 0, nrec = 0;
+  const bool in_step = use >= kInStep;
+  bool more = true;  // slots may be left (the same in every lane of the warp)
+  int mode = AM_IDLE;
+  // the lane's slot; of a path, rec[0] is its first vertex, rec[i] its i-th bounce
+  int pixel = 0, j = 0, m0 = 0, depth = 0, rfm = 0, nrec = 0;
   RmnRng rng;
-  Surf sf;  // the vertex the path stands at
+  Surf sf;  // the vertex the slot stands at
   float3 V, thr, w0;
   float paw = 1.0f, rf = 0.0f, p_rr = 1.0f;
   bool nee = false, exclude = true;
+  int n = 0, cnt = 0;  // light samples taken and to take at the vertex
+  float kf = 1.0f, tot = 0.0f, lwt[8];
   PathAdj acc;
   Record rec[kMaxRecords + 1];
   for (;;) {
-    const unsigned idle = __ballot_sync(FULL, !active);
-    if (more && (__popc(idle) >= kRefill)) {
+    const unsigned idle = __ballot_sync(FULL, mode == AM_IDLE && lane < use);
+    if (more && __popc(idle) >= min(kRefill, use)) {
       unsigned long long base = 0;
       if (lane == 0) base = atomicAdd(next, (unsigned long long)__popc(idle));
       base = __shfl_sync(FULL, base, 0);
       more = (long long)base + __popc(idle) < total;
       const long long t = (long long)base + __popc(idle & ((1u << lane) - 1u));
-      if (!active && t < total) {
+      if (((idle >> lane) & 1u) && t < total) {
         pixel = (int)(t % npx);
-        j = p.spp_d + (int)(t / npx);
+        j = p.slots - 1 - (int)(t / npx);
         const float* gb = gbuf_at(J, pixel);
         if (any_finite3(f3(gb[6], gb[7], gb[8]))) {  // else a miss: sky only, no material
           sf = first_vertex(J, gb);
-          if (j == 0)  // Photo::shade's emission * exposure
-            G.add(sf.id, 4, p.exposure * dot3(dimg_at(J, pixel), sf.emis));
-          rng = rmn_rng(p.seed, (uint32_t)pixel, (uint32_t)j);
-          active = !(len3(sf.emis) > 0.0f) && rng.next() < 1.0f;
-          V = -norm3(sf.pos - p.pos);
-          rf = sf.roughness;
-          rfm = sf.id;
-          sf.eta = 1.0f / sf.eta;
-          depth = 0;
-          nrec = 0;
-          paw = 1.0f;
-          thr = f3(1.0f);
-          acc.S = 0.0f;
-          acc.A_light = acc.A_w0 = acc.dbase = f3(0.0f);
+          m0 = sf.id;
+          if (j == 0) G.add(m0, 4, p.exposure * dot3(dimg_at(J, pixel), sf.emis));  // Photo::shade's emission * exposure
+          if (!(len3(sf.emis) > 0.0f)) {
+            V = -norm3(sf.pos - p.pos);
+            rng = rmn_rng(p.seed, (uint32_t)pixel, (uint32_t)j);
+            if (j < p.spp_d) {
+              mode = AM_FIRST;
+              n = 0;
+              cnt = 1;
+            } else if (rng.next() < 1.0f) {
+              mode = AM_BOUNCE;
+              rf = sf.roughness;
+              rfm = m0;
+              sf.eta = 1.0f / sf.eta;
+              depth = 0;
+              nrec = 0;
+              thr = f3(1.0f);
+              acc.S = 0.0f;
+              acc.A_light = acc.A_w0 = acc.dbase = f3(0.0f);
+            }
+          }
         }
       }
     }
-    if (!__syncthreads_or(active || more)) break;
+    if (in_step ? !__syncthreads_or(mode != AM_IDLE || more) : !__any_sync(FULL, mode != AM_IDLE || more)) break;
     // the bounce from the vertex
     float3 o = f3(0.0f), dir = f3(0.0f);
     bool done = false;  // the path ends in this round
-    if (active) {
+    if (mode == AM_BOUNCE) {
       float3 wv;
       int nf = 0;
       ReflectAD ad;
       sample_reflect(sf, V, rng, dir, wv, nf, &ad);
       if (!any_finite3(dir) || (depth > 0 && depth == p.maxd)) {
-        active = false;  // nothing was added yet: a path's samples come at its end
+        mode = AM_IDLE;  // nothing was added yet: a path's samples come at its end
       } else {
         Record& r = rec[nrec++];
         r.m = sf.id;
@@ -394,7 +352,6 @@ __global__ void __launch_bounds__(kPathThreads, 1)
           w0 = wv;
           paw = nf > 0 ? 1.0f / (float)(1 + nf) : 1.0f;
         } else {
-          wv = wv / 1.0f;
           if (nee) wv = wv / p_rr;
           thr = thr * wv;
           if (nf > 0) paw = paw * (1.0f / (float)(1 + nf));
@@ -404,35 +361,53 @@ __global__ void __launch_bounds__(kPathThreads, 1)
         depth++;
       }
     }
-    __syncthreads();
+    if (in_step) __syncthreads();
+    // the vertex's next light sample
+    const bool sampled = mode == AM_SAMPLE || mode == AM_FIRST;
+    bool go = false;  // it needs a shadow ray
+    float3 ld = f3(0.0f);
+    float aim = 0.0f;
+    LSample ls;
+    int li = -1;
+    if (sampled) {
+      if (n == 0 && s.sky_w == 0 && !light_weights(s, sf, V, lwt, tot)) cnt = 0;
+      if (cnt > 0)
+        go = light_gen(s, sf, V, lwt, tot, mode == AM_FIRST ? p.spp_d : cnt, rng, ld, aim, ls, &li);
+    }
+    if (in_step) __syncthreads();
     float tm;
-    const int h = closest(s, o, dir, tm, active, sh);
-    __syncthreads();
-    // one sample of the path: light, weight, into the path's sums
-    auto add_sample = [&](float3 light, float w) {
-      const float* gb = gbuf_at(J, pixel);
-      DemodAdj d = demod_adj(tweak_base(f3(__ldg(&s.mats[rec[0].m].base))), f3(gb[0], gb[1], gb[2]), w0, light, w,
+    const int h = closest(s, o, dir, tm, mode == AM_BOUNCE, sh);
+    if (in_step) __syncthreads();
+    const bool occ = occluded(s, sf.pos, ld, aim, go, sh, status);
+    if (in_step) __syncthreads();
+    const int drop = J.dropped && mode != AM_IDLE ? J.dropped[pixel] : -1;
+    // a sample's contribution and the path's sums
+    const float* gb = gbuf_at(J, pixel);
+    auto demod = [&](float3 f, float3 light, float w) {
+      DemodAdj d = demod_adj(tweak_base(f3(__ldg(&s.mats[m0].base))), f3(gb[0], gb[1], gb[2]), f, light, w,
                              dimg_at(J, pixel), p.exposure);
       if (!finite1(d.S) || d.S == 0.0f) {
         d.S = 0.0f;
         d.dlight = f3(0.0f);
-        return d;
       }
+      return d;
+    };
+    auto add_path = [&](const DemodAdj& d, float3 light) {
+      if (d.S == 0.0f) return;
       acc.S += d.S;
       acc.A_light += d.dlight * light;
       acc.A_w0 += d.df * w0;
       acc.dbase += d.dbase;
-      return d;
     };
-    int cnt = 0;  // light samples of the vertex, where the path ends there
-    float kf = 1.0f;
-    if (active) {
-      const int drop = J.dropped ? J.dropped[pixel] : -1;
+    if (mode == AM_BOUNCE) {
       if (h == -2) {
         atomicExch(status, 1);
-        active = false;
+        mode = AM_IDLE;
       } else if (h < 0) {
-        if (!exclude && s.sky_w && drop != j * 8) add_sample(sky_get(s, dir) * thr, paw * p.inv_spp);
+        if (!exclude && s.sky_w && drop != j * 8) {
+          const float3 light = sky_get(s, dir) * thr;
+          add_path(demod(w0, light, paw * p.inv_spp), light);
+        }
         done = true;
       } else {
         sf = default_surf();
@@ -448,7 +423,9 @@ __global__ void __launch_bounds__(kPathThreads, 1)
         V = -dir;
         if (len3(sf.emis) > RMN_EPS) {
           if (!exclude && drop != j * 8) {
-            DemodAdj d = add_sample(sf.emis * thr, paw * p.inv_spp);
+            const float3 light = sf.emis * thr;
+            const DemodAdj d = demod(w0, light, paw * p.inv_spp);
+            add_path(d, light);
             G.add(sf.id, 4, d.S);
           }
           done = true;
@@ -457,43 +434,41 @@ __global__ void __launch_bounds__(kPathThreads, 1)
         } else {
           nee = nee && sf.entering;
           if (nee && (depth >= p.maxd || rng.next() > p_rr)) {
+            mode = AM_SAMPLE;
+            n = 0;
             cnt = c_sample_count[depth < 16 ? depth : 16];
+            kf = 1.0f;
             if (depth < p.maxd) kf /= (1.0f - p_rr);
-            done = true;
           }
         }
       }
     }
-    // the light samples of the vertices where paths end
-    if (__syncthreads_or(cnt > 0)) {
-      float lwt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      float tot = 0.0f;
-      if (cnt > 0 && s.sky_w == 0 && !light_weights(s, sf, V, lwt, tot)) cnt = 0;
-      for (int n = 0; __syncthreads_or(n < cnt); ++n) {
-        float3 ld = f3(0.0f);
-        float aim = 0.0f;
-        LSample ls;
-        int li = -1;
-        const bool go = n < cnt && light_gen(s, sf, V, lwt, tot, cnt, rng, ld, aim, ls, &li);
-        __syncthreads();
-        const bool occ = occluded(s, sf.pos, ld, aim, go, sh, status);
-        __syncthreads();
-        if (occ || !go) continue;
-        if ((J.dropped ? J.dropped[pixel] : -1) == j * 8 + n) continue;
-        ls.bsdf *= kf;
-        const float3 light = (ls.light * ls.bsdf) * thr;
-        DemodAdj d = add_sample(light, ls.weight * paw * p.inv_spp);
-        if (d.S == 0.0f) continue;
-        float3 l, q, lr;
-        brdf_logd(sf, V, ld, 2, l, q, lr);
-        const float3 A = d.dlight * light;
-        G.add_base(sf.id, A * l - d.S * q);
-        G.add(rfm, 3, dot3(A, lr));
-        if (li >= 0) G.add(__ldg(&s.lights[li].material), 4, d.S);
+    if (in_step) __syncthreads();
+    if (sampled) {
+      const bool first = mode == AM_FIRST;
+      if (go && !occ && (first || drop != j * 8 + n)) {
+        if (!first) ls.bsdf *= kf;
+        const float3 light = first ? ls.light : (ls.light * ls.bsdf) * thr;
+        const DemodAdj d = demod(first ? ls.bsdf : w0, light, first ? ls.weight : ls.weight * paw * p.inv_spp);
+        if (d.S != 0.0f) {
+          if (!first) add_path(d, light);
+          float3 l, q, lr;
+          brdf_logd(sf, V, ld, 2, l, q, lr);
+          const float3 A = first ? d.df * ls.bsdf : d.dlight * light;
+          float3 gbase = A * l - d.S * q;
+          if (first) gbase += d.dbase;
+          G.add_base(sf.id, gbase);
+          G.add(first ? sf.id : rfm, 3, dot3(A, lr));
+          if (li >= 0) G.add(__ldg(&s.lights[li].material), 4, d.S);
+        }
+      }
+      if (++n >= cnt) {
+        done = !first;
+        mode = AM_IDLE;
       }
     }
     if (done) {
-      active = false;
+      mode = AM_IDLE;
       if (acc.S != 0.0f) {
         for (int i = 1; i < nrec; ++i) {
           const Record& r = rec[i];
@@ -506,7 +481,10 @@ __global__ void __launch_bounds__(kPathThreads, 1)
       }
     }
   }
-  grad_end(G, nmats);
+  __syncthreads();
+  if (use_sh)
+    for (int i = threadIdx.x; i < nmats * kGradPerMat; i += kPathThreads)
+      if (sg[i] != 0.0f) atomicAdd(gout + i, (double)sg[i]);
 }
 
 __global__ void to_float_kernel(const double* in, float* out, int n) {
@@ -534,27 +512,17 @@ rmn_status launch_adjoint(const rmn_scene* scene, const rmn_render_args& args, c
   unsigned long long* next = reinterpret_cast<unsigned long long*>(acc + ng);
   int* status = reinterpret_cast<int*>(next + 1);
   e = cudaMemsetAsync(acc, 0, (size_t)ng * sizeof(double) + 16, st);
-  const long long npx = (long long)J.p.W * J.p.H;
-  const long long lights = npx * J.p.spp_d, paths = npx * (J.p.slots - J.p.spp_d);
+  const long long total = (long long)J.p.W * J.p.H * J.p.slots;
   const size_t shared =
       sizeof(AdjTrav) * (kPathThreads / 32) + (nmats <= kSharedMats ? (size_t)ng * sizeof(float) : 0);
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // as many blocks as the device holds, or as the slots need
-  auto blocks = [&](const void* kernel, int threads, size_t shared, long long slots) {
-    int per_sm = 0;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, shared);
-    return (unsigned)std::min<long long>((slots + threads - 1) / threads, (long long)sms * std::max(per_sm, 1));
-  };
-  if (e == cudaSuccess && lights > 0) {
-    const unsigned g = blocks((const void*)adjoint_light_kernel, kPathThreads, shared, lights);
-    if (e == cudaSuccess) adjoint_light_kernel<<<g, kPathThreads, shared, st>>>(J, lights, nmats, acc, status);
-  }
-  if (e == cudaSuccess && paths > 0) {
-    const unsigned g = blocks((const void*)adjoint_path_kernel, kPathThreads, shared, paths);
-    if (e == cudaSuccess) adjoint_path_kernel<<<g, kPathThreads, shared, st>>>(J, paths, nmats, acc, next, status);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+  if (e == cudaSuccess && total > 0) {
+    // the slots over all warps first, then over their lanes
+    const long long blocks = (long long)kPathBlocks * device_sms(), warps = blocks * (kPathThreads / 32);
+    const int use = (int)std::min<long long>(32, (total + warps - 1) / warps);
+    const long long per_block = (long long)use * (kPathThreads / 32);
+    const unsigned grid = (unsigned)std::min<long long>(blocks, (total + per_block - 1) / per_block);
+    adjoint_kernel<<<grid, kPathThreads, shared, st>>>(J, total, use, nmats, acc, next, status);
   }
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) {
