@@ -20,17 +20,15 @@ namespace {
 
 // STACK: shared stack entries (RMN_STACK_SMALL for trees that fit it: one
 // more block per SM). use: lanes of a warp that take rays (the others help
-// with the leaves).
-template <bool SHADOW, int STACK>
+// with the leaves). COUNTED: lanes take rays from the counter `next` as they
+// become free; else there is a lane for every ray, and each warp takes its own.
+template <bool SHADOW, int STACK, bool COUNTED>
 __global__ void __launch_bounds__(128, RMN_COOP_BLOCKS(STACK)) trace_kernel(DevScene s, const float4* __restrict__ rays, int64_t n,
                                                     float4* __restrict__ hits, uint8_t* __restrict__ occ,
                                                     unsigned long long* __restrict__ next, int* status, int use) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   bool active = false, retired = lane >= use;
-  // without a counter: each warp its own `use` rays
-  const unsigned long long first = (unsigned long long)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * use;
-  bool fetched = false;
   int64_t i = 0;
   TRay r;
   float tmin = 0.0f, aim = 0.0f, restart = 0.0f;
@@ -50,10 +48,9 @@ __global__ void __launch_bounds__(128, RMN_COOP_BLOCKS(STACK)) trace_kernel(DevS
     if (need) {
       const int leader = __ffs(need) - 1;
       unsigned long long base = 0;
-      if (!next) base = fetched ? (unsigned long long)n : first;
+      if (!COUNTED) base = (unsigned long long)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * use;
       else if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(need));
-      fetched = true;
-      base = __shfl_sync(0xffffffffu, base, leader);
+      if (COUNTED) base = __shfl_sync(0xffffffffu, base, leader);
       if (!active && !retired) {
         i = (int64_t)(base + __popc(need & lt));
         if (i < n) {
@@ -95,12 +92,13 @@ __global__ void __launch_bounds__(128, RMN_COOP_BLOCKS(STACK)) trace_kernel(DevS
       hits[i] = make_float4(a.w, t.tmax, bc.y, bc.z);
     }
     active = false;
+    if (!COUNTED) retired = true;
   }
 }
 
 // Occlusion queries of a scene without alpha-tested materials: pending
 // leaves, order-free (trace.cuh, occ_nodes / occ_leaves).
-template <int STACK>
+template <int STACK, bool COUNTED>
 __global__ void __launch_bounds__(128, RMN_OCC_BLOCKS) occ_kernel(DevScene s, const float4* __restrict__ rays,
                                                                           int64_t n, uint8_t* __restrict__ occ,
                                                                           unsigned long long* __restrict__ next,
@@ -108,9 +106,6 @@ __global__ void __launch_bounds__(128, RMN_OCC_BLOCKS) occ_kernel(DevScene s, co
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   bool active = false, retired = lane >= use;
-  // without a counter: each warp its own `use` rays
-  const unsigned long long first = (unsigned long long)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * use;
-  bool fetched = false;
   int64_t i = 0;
   TRay r;
   float aim = 0.0f;
@@ -124,10 +119,9 @@ __global__ void __launch_bounds__(128, RMN_OCC_BLOCKS) occ_kernel(DevScene s, co
     if (need) {
       const int leader = __ffs(need) - 1;
       unsigned long long base = 0;
-      if (!next) base = fetched ? (unsigned long long)n : first;
+      if (!COUNTED) base = (unsigned long long)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * use;
       else if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(need));
-      fetched = true;
-      base = __shfl_sync(0xffffffffu, base, leader);
+      if (COUNTED) base = __shfl_sync(0xffffffffu, base, leader);
       if (!active && !retired) {
         i = (int64_t)(base + __popc(need & lt));
         if (i < n) {
@@ -149,6 +143,7 @@ __global__ void __launch_bounds__(128, RMN_OCC_BLOCKS) occ_kernel(DevScene s, co
     if (st == -2) atomicExch(status, (int)rmn::kDevStackOverflow);
     occ[i] = (o && st != -2) ? 1 : 0;
     active = false;
+    if (!COUNTED) retired = true;
   }
 }
 
@@ -157,7 +152,7 @@ cudaError_t launch_kernel(const DevScene& s, const float4* rays, int64_t n, floa
                           cudaStream_t stream) {
   const int threads = 128;
   const bool order_free = SHADOW && !s.has_alpha;
-  const void* kernel = order_free ? (const void*)occ_kernel<STACK> : (const void*)trace_kernel<SHADOW, STACK>;
+  const void* kernel = order_free ? (const void*)occ_kernel<STACK, true> : (const void*)trace_kernel<SHADOW, STACK, true>;
   int blocks = rmn::device_sms() * rmn::blocks_per_sm(kernel, threads);
   // the rays go over all the warps the device holds, `use` of a warp's lanes
   // taking one each: a warp's time is its rays' divergent steps one after the
@@ -171,8 +166,8 @@ cudaError_t launch_kernel(const DevScene& s, const float4* rays, int64_t n, floa
   if (need <= blocks) {
     // every ray has its lane: no counter to hand them out
     blocks = (int)need;
-    if (order_free) occ_kernel<STACK><<<blocks, threads, 0, stream>>>(s, rays, n, occ, nullptr, status, use);
-    else trace_kernel<SHADOW, STACK><<<blocks, threads, 0, stream>>>(s, rays, n, hits, occ, nullptr, status, use);
+    if (order_free) occ_kernel<STACK, false><<<blocks, threads, 0, stream>>>(s, rays, n, occ, nullptr, status, use);
+    else trace_kernel<SHADOW, STACK, false><<<blocks, threads, 0, stream>>>(s, rays, n, hits, occ, nullptr, status, use);
     return cudaGetLastError();
   }
   unsigned long long* next = nullptr;
@@ -180,8 +175,8 @@ cudaError_t launch_kernel(const DevScene& s, const float4* rays, int64_t n, floa
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(next, 0, sizeof(unsigned long long), stream);
   if (e == cudaSuccess) {
-    if (order_free) occ_kernel<STACK><<<blocks, threads, 0, stream>>>(s, rays, n, occ, next, status, use);
-    else trace_kernel<SHADOW, STACK><<<blocks, threads, 0, stream>>>(s, rays, n, hits, occ, next, status, use);
+    if (order_free) occ_kernel<STACK, true><<<blocks, threads, 0, stream>>>(s, rays, n, occ, next, status, use);
+    else trace_kernel<SHADOW, STACK, true><<<blocks, threads, 0, stream>>>(s, rays, n, hits, occ, next, status, use);
     e = cudaGetLastError();
   }
   const cudaError_t f = cudaFreeAsync(next, stream);
