@@ -864,7 +864,7 @@ rmn_status rmn_batch_autotune(const rmn_batch_item* items, int32_t n, float pixe
     const int proxy_pool =
         (int)std::max<double>(4096.0, std::round((cp > 0 ? cp : kDefaultPoolWorkers) * f / 128.0) * 128.0);
     BatchState* b = nullptr;
-    r = batch_create(its.data(), n, true, proxy_pool, cl, ck, co, st, &b);
+    r = batch_create(its.data(), n, true, proxy_pool, cl, ck, co, st, &b, f);
     if (r != RMN_OK) break;
     r = batch_launch(b, st);  // warm-up
     if (r == RMN_OK) {

@@ -1808,6 +1808,7 @@ struct BatchState {
   bool tex = false;           // some job's scene has textures
   bool shallow = true;        // the traversal runs its RMN_STACK_SMALL-entry build
   bool direct = false;        // few units: block_kernel renders them all, without wavefront iterations
+  long long tail = 0;         // workers with which block_kernel takes the end of a longer render
   Pool pool[kMaxLanes] = {};  // each lane's share of the worker arrays
   Queues q[kMaxLanes] = {};
   // ray binning (ray_order): per lane, the reordered closest and shadow
@@ -2122,7 +2123,7 @@ static rmn_status run(BatchState* b, cudaStream_t st, Counters* ctr, cudaEvent_t
       waiting[l] = (long long)h.lane[l].q[1].c + h.lane[l].q[1].sd + h.lane[l].q[1].nw;
       live += (unsigned)waiting[l];
     }
-    if (drain && live > 0 && (long long)live <= block_capacity() &&
+    if (drain && live > 0 && (long long)live <= b->tail &&
         (long long)h.next_unit >= b->table.total_units) {
       e = launch_blocks(b, waiting, st);
       if (e != cudaSuccess) return cuda_fail(e, "render tail");
@@ -2237,7 +2238,7 @@ int default_stack_entries(const RenderItem* items, int n) {
 }
 
 rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int pool_workers, int lanes,
-                        int stack_entries, int ray_order, cudaStream_t st, BatchState** out) {
+                        int stack_entries, int ray_order, cudaStream_t st, BatchState** out, double proxy_of) {
   *out = nullptr;
   // the traversal stack must hold every item's deepest path of deferred
   // children; a larger one only costs occupancy
@@ -2258,12 +2259,15 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
   b->table.slots = S_def;
   b->use_graph = use_graph;
   b->binned = ray_order != 0;
-  b->lanes = lanes > 0 ? std::min(lanes, kMaxLanes) : default_lanes(b->table.total_units);
+  b->lanes = lanes > 0 ? std::min(lanes, kMaxLanes)
+                       : default_lanes((long long)((double)b->table.total_units / proxy_of));
   // workers per lane; no more lanes and workers than there are units, nor, for a
   // render without wavefront, than are resident; the default pool halves while
   // the workers would take more than a quarter of the free device memory
   long long per = pool_workers > 0 ? pool_workers : kDefaultPoolWorkers;
-  b->direct = b->table.total_units <= kDirectUnits;
+  // a proxy of a larger batch is rendered as that batch would be
+  b->direct = (double)b->table.total_units <= proxy_of * (double)kDirectUnits;
+  b->tail = (long long)(proxy_of * (double)block_capacity());
   if (b->direct) {
     b->lanes = 1;
     per = std::min(per, std::min(block_capacity(), b->table.total_units));

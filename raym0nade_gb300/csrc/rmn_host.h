@@ -160,8 +160,9 @@ void noalloc_forget_addresses();
 // or RMN_STACK entries (0: the smallest that holds every item's tree).
 // ray_order: 1 bins each ray queue by origin cell and direction octant
 // before it is traced, 0 traces the queues in the order they were filled.
+// proxy_of: the batch stands for one 1 / proxy_of times its size (autotuner).
 rmn_status batch_create(const RenderItem* items, int n, bool use_graph, int pool_workers, int lanes,
-                        int stack_entries, int ray_order, cudaStream_t st, BatchState** out);
+                        int stack_entries, int ray_order, cudaStream_t st, BatchState** out, double proxy_of = 1.0);
 // The traversal stack the library picks for these items (RMN_STACK_SMALL when
 // every tree is at most RMN_STACK_SMALL - 1 deep, else RMN_STACK).
 int default_stack_entries(const RenderItem* items, int n);
