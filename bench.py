@@ -53,7 +53,8 @@ FALLBACK_HBM_GBS = 6800.0
 # launch configurations given beside them, summed from ncu captures (metrics
 # dram__bytes_read.sum, dram__bytes_write.sum, lts__t_bytes.sum) of
 #   python bench.py --profile-case batch --slots 2 --pool 8388608 --lanes L --stack S
-# (ncu cannot run inside the timed region). The line takes the capture of
+# (ncu cannot run inside the timed region; captured before the box tests were
+# paired, which left every visit as it was). The line takes the capture of
 # the timed configuration, and says so, or else the first and says that.
 BATCH64_TRAVERSAL_BYTES = [
     {"config": {"slots_per_unit": 2, "pool_workers": 1 << 23, "lanes": 3, "stack_entries": 23, "ray_order": 0},
@@ -747,9 +748,9 @@ def run_gpu(args, rank, world, dist):
               "source": "ncu lts__t_bytes.sum over the same launches; copy_rate: a device copy between two "
                         "L2-resident 24 MiB buffers, measured here"}
     limiter = ("instruction issue and dependent-load latency: in steady state (ncu) the closest-hit traversal "
-               "uses 67 % of its issue slots with 17.5 of 32 lanes active per instruction (warp-cooperative "
-               "leaves), the occlusion traversal 69 % with 18.5 lanes (pending leaves), both stalled mostly on "
-               "L1/L2 loads (long scoreboard 3.1-3.9 per issue) and fixed-latency dependencies (2.3-2.9); their "
+               "uses 63 % of its issue slots with 19.5 of 32 lanes active per instruction (warp-cooperative "
+               "leaves), the occlusion traversal 68 % with 20.2 lanes (pending leaves), both stalled mostly on "
+               "L1/L2 loads (long scoreboard 4.1 per issue) and fixed-latency dependencies (2.4-2.5); their "
                "measured DRAM traffic is a small share of the algorithmic bytes (L1/L2 hits) and neither DRAM "
                "nor L2 runs near its rate")
     base, _ = cpu_baseline(insts) if args.cpu_baseline else (None, None)
@@ -758,8 +759,9 @@ def run_gpu(args, rank, world, dist):
         "ms_per_step": ms_b, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic (seeded procedural scenes; no dataset)",
         "config": workload_config(insts, desc, world),
-        "setup": {"launch": "rmn_batch: G-buffer kernel, then wavefront iterations (shade, NEE, slot, closest and "
-                            "shadow traversal kernels) of every lane as parallel branches of a replayed CUDA graph",
+        "setup": {"launch": "rmn_batch: G-buffer kernel, then wavefront iterations (shade, bounce, NEE, slot, light, path, "
+                            "closest and shadow traversal kernels) of every lane as parallel branches of a replayed CUDA "
+                            "graph; the last workers in block_kernel",
                   "scene_bytes": scene_bytes, "scene_build_s": round(build_s, 1)},
         "plain": {"value": plain, "unit": UNIT, "ms_per_step": ms_p, "launches_per_step": 2 * len(insts),
                   "batched_over_plain": value / plain},

@@ -380,9 +380,9 @@ rmn_status rmn_fxaa(const float* rgb_in, float* rgb_out, int32_t width, int32_t 
  * Photo::shade(options), then the depth-of-field blur (RMN_SHADE_DEPTH_OF_FIELD,
  * src/image.cpp:282-356) and bloom (RMN_SHADE_BLOOM, :248-280) when asked,
  * gammaCorrection when RMN_SHADE_GAMMA is set (postProcessing always applies
- * it), FXAA last -> rgb (3 floats per pixel). The depth-of-field blur sorts
- * the pixels' depths on the host (std::stable_sort, as the reference) and
- * synchronises the stream once. */
+ * it), FXAA last -> rgb (3 floats per pixel). The depth-of-field blur takes
+ * the pixels in the order std::stable_sort gives their depths, as the
+ * reference, found on the device; the host waits for the stream to size it. */
 rmn_status rmn_post_process(const rmn_image* image, const rmn_post_args* args, int32_t options, float* rgb,
                             void* stream);
 

@@ -1286,7 +1286,7 @@ __global__ void __launch_bounds__(128, RMN_OCC_BLOCKS) qocc_kernel(const Job* __
 // kind: the steps' code is far larger than an SM's instruction caches, and with
 // tasks of all kinds side by side (three blocks of 256 threads per SM) a warp
 // waited 17 of 45 cycles between two issues for its instructions (Cornell
-// 256x256, 64 spp, all in this kernel: 12.9 ms against 4.5). Only when a stage
+// 256x256, 64 spp, all in this kernel: 12.9 ms against 5.2). Only when a stage
 // has no more tasks than the block has warps do they run side by side, cut to
 // fewer entries where that gives the idle warps work: then the longest of
 // them, not their sum, is what a round takes.
