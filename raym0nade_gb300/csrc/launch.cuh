@@ -9,7 +9,8 @@
 // one implies the end of all before it. Used where the predecessor is a
 // kernel of this library in the same stream.
 //
-// No kernel lets its successor start before its own blocks have ended
+// Only where one chain of kernels has the device to itself: see follow() in
+// render.cu. No kernel lets its successor start before its own blocks have ended
 // (griddepcontrol.launch_dependents): waiting blocks hold the slots that the
 // other lanes' kernels would run in (1080p terrain, 64 spp: 57.0 -> 59.5 ms;
 // ten renders in a batch 12.1 -> 12.8).

@@ -1899,13 +1899,15 @@ static cudaError_t launch_init(BatchState* b, cudaStream_t st, Counters* ctr) {
   return cudaGetLastError();
 }
 
-// One kernel of an iteration after another (launch.cuh). Against launches that
-// start when the kernel before has ended: Cornell 256x256, 64 spp: 4.22 -> 4.00 ms;
-// glass 250x250, 16 spp: 7.50 -> 7.20; textured 640x480, 32 spp: 7.19 -> 7.09; a
-// 1080p terrain and ten renders in a batch, whose kernels are long, unchanged.
+// One kernel of an iteration after another. In a render of one lane its launch
+// overlaps the end of the kernel before (launch.cuh): Cornell 256x256, 64 spp:
+// 4.22 -> 4.00 ms; glass 250x250, 16 spp: 7.50 -> 7.20. With several lanes the
+// others' kernels fill that gap, and the blocks that wait hold their slots: 64
+// renders of 128^2 to 1024^2 one by one 910 -> 960 ms.
 template <class... P, class... A>
-static void follow(void (*kernel)(P...), int blocks, cudaStream_t st, A... args) {
-  launch_after(kernel, dim3((unsigned)blocks), dim3(128), 0, st, args...);
+static void follow(const BatchState* b, void (*kernel)(P...), int blocks, cudaStream_t st, A... args) {
+  if (b->lanes == 1) launch_after(kernel, dim3((unsigned)blocks), dim3(128), 0, st, args...);
+  else kernel<<<blocks, 128, 0, st>>>(static_cast<P>(args)...);
 }
 
 // The two traversal kernels of an iteration (closest, then shadow), on as
@@ -1915,14 +1917,14 @@ static void launch_qtrace(BatchState* b, const Pool& P, const Queues& Q, Ctl* ct
                           cudaStream_t st) {
   int tb = device_sms() * blocks_per_sm(qtrace_kernel<false, COUNT, ALPHA, STACK>);
   if (tb > lb) tb = lb;
-  follow(qtrace_kernel<false, COUNT, ALPHA, STACK>, tb, st, b->d_jobs, P, Q, ctl, par, b->d_status, ctr);
+  follow(b, qtrace_kernel<false, COUNT, ALPHA, STACK>, tb, st, b->d_jobs, P, Q, ctl, par, b->d_status, ctr);
   // the shadow queue: ordered search with the alpha-test retry, else order-free occlusion
   if constexpr (ALPHA) {
-    follow(qtrace_kernel<true, COUNT, ALPHA, STACK>, tb, st, b->d_jobs, P, Q, ctl, par, b->d_status, ctr);
+    follow(b, qtrace_kernel<true, COUNT, ALPHA, STACK>, tb, st, b->d_jobs, P, Q, ctl, par, b->d_status, ctr);
   } else {
     int ob = device_sms() * blocks_per_sm(qocc_kernel<COUNT, STACK>);
     if (ob > lb) ob = lb;
-    follow(qocc_kernel<COUNT, STACK>, ob, st, b->d_jobs, P, Q, ctl, par, b->d_status, ctr);
+    follow(b, qocc_kernel<COUNT, STACK>, ob, st, b->d_jobs, P, Q, ctl, par, b->d_status, ctr);
   }
 }
 
@@ -1941,18 +1943,18 @@ static cudaError_t launch_iteration(BatchState* b, int lane, cudaStream_t st, Co
   const int sms = device_sms();
   const int gs = sms * blocks_per_sm(shade_kernel), gn = sms * blocks_per_sm(nee_kernel);
   // the first iteration of a chunk follows a copy, a fork or another graph
-  if (k > 0) follow(shade_kernel, gs, st, b->d_jobs, P, Q, ctl, par, b->d_parts, b->d_status);
+  if (k > 0) follow(b, shade_kernel, gs, st, b->d_jobs, P, Q, ctl, par, b->d_parts, b->d_status);
   else shade_kernel<<<gs, 128, 0, st>>>(b->d_jobs, P, Q, ctl, par, b->d_parts, b->d_status);
-  follow(bounce_kernel, sms * blocks_per_sm(bounce_kernel), st, b->d_jobs, P, Q, ctl, par);
-  follow(nee_kernel, gn, st, b->d_jobs, P, Q, ctl, par, b->d_parts);
-  follow(slot_kernel, sms * blocks_per_sm(slot_kernel), st, b->d_jobs, nj, P, Q, ctl, &b->d_ctl->next_unit, par,
+  follow(b, bounce_kernel, sms * blocks_per_sm(bounce_kernel), st, b->d_jobs, P, Q, ctl, par);
+  follow(b, nee_kernel, gn, st, b->d_jobs, P, Q, ctl, par, b->d_parts);
+  follow(b, slot_kernel, sms * blocks_per_sm(slot_kernel), st, b->d_jobs, nj, P, Q, ctl, &b->d_ctl->next_unit, par,
                b->table.total_units, b->d_parts);
   if (ctr) {
-    follow(light_kernel<true>, sms * blocks_per_sm(light_kernel<true>), st, b->d_jobs, P, Q, ctl, par, ctr);
-    follow(path_kernel<true>, sms * blocks_per_sm(path_kernel<true>), st, b->d_jobs, P, Q, ctl, par, ctr);
+    follow(b, light_kernel<true>, sms * blocks_per_sm(light_kernel<true>), st, b->d_jobs, P, Q, ctl, par, ctr);
+    follow(b, path_kernel<true>, sms * blocks_per_sm(path_kernel<true>), st, b->d_jobs, P, Q, ctl, par, ctr);
   } else {
-    follow(light_kernel<false>, sms * blocks_per_sm(light_kernel<false>), st, b->d_jobs, P, Q, ctl, par, ctr);
-    follow(path_kernel<false>, sms * blocks_per_sm(path_kernel<false>), st, b->d_jobs, P, Q, ctl, par, ctr);
+    follow(b, light_kernel<false>, sms * blocks_per_sm(light_kernel<false>), st, b->d_jobs, P, Q, ctl, par, ctr);
+    follow(b, path_kernel<false>, sms * blocks_per_sm(path_kernel<false>), st, b->d_jobs, P, Q, ctl, par, ctr);
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (ev) cudaEventRecord(ev[1], st);
