@@ -257,6 +257,11 @@ constexpr int kRefill = 4;
 // instructions fit side by side and a barrier only makes the short wait for the
 // long (24x24, 4 spp: 202 us without barriers, 230 with).
 constexpr int kInStep = 4;
+// Slots a lane takes one after the other before a warp uses more lanes: most
+// slots end long before the longest, so a lane that refills fills the time its
+// warp runs anyway, and fewer lanes diverge less. 64x64, 16 spp: 622, 584 and 594 us
+// with 1, 3 and 4 (6: 684); 96x96, 16 spp: 628, 603 and 635; 256x256, 32 spp the same.
+constexpr int kTurns = 3;
 enum AdjMode { AM_IDLE = 0, AM_BOUNCE, AM_SAMPLE, AM_FIRST };
 
 // total: all slots of all pixels; use: lanes of a warp that take slots, fewer
@@ -517,9 +522,12 @@ rmn_status launch_adjoint(const rmn_scene* scene, const rmn_render_args& args, c
       sizeof(AdjTrav) * (kPathThreads / 32) + (nmats <= kSharedMats ? (size_t)ng * sizeof(float) : 0);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
   if (e == cudaSuccess && total > 0) {
-    // the slots over all warps first, then over their lanes
+    // the slots over all warps first (kInStep lanes), then over their lanes, kTurns to
+    // a lane before it takes more lanes
     const long long blocks = (long long)kPathBlocks * device_sms(), warps = blocks * (kPathThreads / 32);
-    const int use = (int)std::min<long long>(32, (total + warps - 1) / warps);
+    const long long each = (total + warps - 1) / warps;
+    const int use = (int)std::min<long long>(
+        32, std::max(std::min<long long>(each, kInStep), (each + kTurns - 1) / kTurns));
     const long long per_block = (long long)use * (kPathThreads / 32);
     const unsigned grid = (unsigned)std::min<long long>(blocks, (total + per_block - 1) / per_block);
     adjoint_kernel<<<grid, kPathThreads, shared, st>>>(J, total, use, nmats, acc, next, status);
