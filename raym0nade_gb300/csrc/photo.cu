@@ -463,7 +463,9 @@ __global__ void __launch_bounds__(kCandThreads) dof_candidates_kernel(
 // A receiver that has gained so much that no weight of at least eps can be
 // added any more (0.99 - gained below eps / 2; a candidate's weight is at least
 // eps or skipped, and what is left of it after the cap is below eps, so it is
-// skipped) is done, and a block whose receivers are all done stops.
+// skipped) is done, and a block whose receivers are all done stops. Not so a
+// receiver whose own weight is NaN (a pixel without a hit): that weight is not
+// skipped and reaches itself alone, so it waits for its own turn.
 constexpr int kFoldThreads = 256;
 constexpr int kFoldChunk = 128;
 
@@ -488,7 +490,12 @@ __global__ void __launch_bounds__(kFoldThreads) dof_fold_kernel(
   float gained = 0.0f;
 #pragma unroll
   for (int m = 0; m < NI; ++m) blur[m] = f3(0.0f);
-  bool done = !receiver;
+  bool done = !receiver, fills = false;
+  if (receiver) {
+    const float4 own = src[(size_t)(y0 + ry) * W + x0 + rx];
+    const float w = (1.0f < own.x ? 1.0f : own.x) / own.y;
+    fills = w == w;
+  }
   for (int k0 = 0; k0 < n; k0 += kFoldChunk) {
     if (__syncthreads_and(done)) break;
     const int len = min(kFoldChunk, n - k0);
@@ -540,7 +547,7 @@ __global__ void __launch_bounds__(kFoldThreads) dof_fold_kernel(
         }
         gained += w;
       }
-      done = done || 0.99f - gained < 0.5f * RMN_EPS;
+      done = done || (fills && 0.99f - gained < 0.5f * RMN_EPS);
     }
   }
   if (!receiver) return;

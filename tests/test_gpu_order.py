@@ -29,3 +29,24 @@ def test_nan_depth_order(port, w, h, nan):
     got = np_(ph.post_process(api.Full | api.DoDepthFieldBlur))
     _, want = port.photo(rec, 8, api.Full | api.DoDepthFieldBlur, **post)
     assert np.array_equal(got, want, equal_nan=True)
+
+
+def test_a_pixel_without_a_hit_is_reached_when_full(port):
+    """A pixel without a hit gets its own NaN colour, however much weight its
+    neighbours have given it before its turn in the order: beside a near wall,
+    blurred wide, the far one's pixels receive more than the 0.99 they take."""
+    w, h = 96, 80
+    rec = photo_records(w, h, 3)
+    r = rec.reshape(-1, 40)
+    rng = np.random.default_rng(1)
+    x = np.arange(w * h) % w
+    r[:, 22:24] = 0.0
+    r[:, 24] = np.where(x < w // 2, 0.3, 2.0) + 1e-3 * rng.random(w * h)
+    miss = (np.abs(x - w // 2 - 4) < 8) & (rng.random(w * h) < 0.04)
+    r[miss, 22:25] = np.nan
+    post = dict(PHOTO_POST, coc=10.0)
+    ph = photo_from_records(rec, post)
+    got = np_(ph.post_process(api.Full | api.DoDepthFieldBlur))
+    _, want = port.photo(rec, 8, api.Full | api.DoDepthFieldBlur, **post)
+    assert np.isnan(want).any(-1).sum() == miss.sum()
+    assert np.array_equal(got, want, equal_nan=True)
