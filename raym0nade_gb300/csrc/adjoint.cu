@@ -51,8 +51,8 @@ struct AdjJob {
   const float* dimg;  // dL/dI, 3 per pixel
 };
 
-// Gradient accumulation: a block-wide table in shared memory, flushed to the
-// double-precision global table when the block ends.
+// Gradient accumulation: a block-wide table in shared memory, added to the
+// double-precision global table every kFlushRounds rounds and when the block ends.
 struct GradSink {
   float* sh;
   double* gl;
@@ -262,6 +262,15 @@ constexpr int kInStep = 4;
 // warp runs anyway, and fewer lanes diverge less. 64x64, 16 spp: 622, 584 and 594 us
 // with 1, 3 and 4 (6: 684); 96x96, 16 spp: 628, 603 and 635; 256x256, 32 spp the same.
 constexpr int kTurns = 3;
+// Rounds after which a block adds its table, in 32 bits, to the double-precision
+// sums: a part then holds some 170 slots however large the render (with fewer than
+// kInStep lanes a warp a block has some two dozen slots in all, and its table is added
+// once, at the end). At 512x512, 256 spp, 220,000 slots a block, one part a block put
+// the gradient up to 4.3e-6 of it from the sum of its bands'; parts of 1, 2, 4 and 8
+// rounds leave the rounding of the result alone (5e-8). 256x256, 32 spp, 16
+// materials: 2986 us with one part, 2978, 2989, 2989 and 3002; 2048 materials 3064,
+// 3109, 3092, 3084 and 3069.
+constexpr int kFlushRounds = 2;
 enum AdjMode { AM_IDLE = 0, AM_BOUNCE, AM_SAMPLE, AM_FIRST };
 
 // total: all slots of all pixels; use: lanes of a warp that take slots, fewer
@@ -273,14 +282,21 @@ __global__ void __launch_bounds__(kPathThreads, kPathBlocks)
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   AdjTrav& sh = reinterpret_cast<AdjTrav*>(adj_shared)[threadIdx.x >> 5];
-  // the block's gradient table, where it fits, flushed to the double-precision
-  // sums at the end
+  // the block's gradient table, where it fits
   float* sg = reinterpret_cast<float*>(adj_shared + sizeof(AdjTrav) * (kPathThreads / 32));
   const bool use_sh = nmats <= kSharedMats;
   if (use_sh)
     for (int i = threadIdx.x; i < nmats * kGradPerMat; i += kPathThreads) sg[i] = 0.0f;
   __syncthreads();
   GradSink G{sg, gout, use_sh};
+  auto flush = [&] {
+    for (int i = threadIdx.x; i < nmats * kGradPerMat; i += kPathThreads)
+      if (sg[i] != 0.0f) {
+        atomicAdd(gout + i, (double)sg[i]);
+        sg[i] = 0.0f;
+      }
+  };
+  int rounds = 0;
   const Params& p = J.p;
   const DevScene& s = J.s;
   const long long npx = (long long)p.W * p.H;
@@ -337,6 +353,8 @@ __global__ void __launch_bounds__(kPathThreads, kPathBlocks)
       }
     }
     if (in_step ? !__syncthreads_or(mode != AM_IDLE || more) : !__any_sync(FULL, mode != AM_IDLE || more)) break;
+    // here every add of the rounds before is done, and the next follows a barrier
+    if (in_step && use_sh && ++rounds % kFlushRounds == 0) flush();
     // the bounce from the vertex
     float3 o = f3(0.0f), dir = f3(0.0f);
     bool done = false;  // the path ends in this round
@@ -487,9 +505,7 @@ __global__ void __launch_bounds__(kPathThreads, kPathBlocks)
     }
   }
   __syncthreads();
-  if (use_sh)
-    for (int i = threadIdx.x; i < nmats * kGradPerMat; i += kPathThreads)
-      if (sg[i] != 0.0f) atomicAdd(gout + i, (double)sg[i]);
+  if (use_sh) flush();
 }
 
 __global__ void to_float_kernel(const double* in, float* out, int n) {

@@ -276,3 +276,30 @@ def test_c5_all_parameters_against_central_differences():
     tol = 0.02 * np.abs(mf) + 4.0 * se + 1e-3 * np.abs(mf).max()
     print("roughness adjoint", np.round(ma, 1), "differences", np.round(mf, 1), "standard error", np.round(se, 1))
     assert (np.abs(ma - mf) <= tol).all(), np.c_[ma, mf, se]
+
+
+def test_gradient_is_the_sum_of_its_parts():
+    """The gradient is linear in dL/dI, and the replay of a pixel does not
+    depend on its neighbours' dL/dI: with a mask of ones and zeros the parts'
+    contributions are the whole's, number for number. So the gradient of the
+    whole image is the sum of the gradients of its bands, up to the rounding of
+    each result to 32 bits (2^-24 of it) and that of the sums inside (1e-9: some
+    hundred 32-bit additions to a part round it by 2e-7 or so, independently in
+    each of the 100,000 parts that are added in double precision). 512 x 512, 256
+    spp: 67 M sample slots, some 220,000 in each of the kernel's blocks."""
+    w, spp, bands = 512, 256, 8
+    m = api.Model(scenes.cornell16())
+    a = api.RenderArgs.from_camera(scenes.cornell_camera(w, w, spp), seed=3)
+    ph = api.render(m, a)
+    whole = api.adjoint(m, a, ph, torch.ones(w * w, 3, device="cuda")).cpu().numpy().astype(np.float64)
+    parts = []
+    for k in range(bands):
+        d = torch.zeros(bands, w * w // bands, 3, device="cuda")
+        d[k] = 1.0
+        parts.append(api.adjoint(m, a, ph, d.reshape(-1, 3)).cpu().numpy().astype(np.float64))
+    parts = np.array(parts)
+    tol = 2.0 ** -24 * (np.abs(whole) + np.abs(parts).sum(0)) + 1e-9 * np.abs(whole)
+    cols = [0, 1, 2, 4]  # base colour and emission: every contribution is positive
+    err = np.abs(whole - parts.sum(0))
+    print("largest relative difference", (err / np.maximum(np.abs(whole), 1e-30))[:, cols].max())
+    assert (err <= tol)[:, cols].all(), (err / np.maximum(tol, 1e-30))[:, cols]
