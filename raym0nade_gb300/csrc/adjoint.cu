@@ -534,9 +534,13 @@ rmn_status launch_adjoint(const rmn_scene* scene, const rmn_render_args& args, c
   int* status = reinterpret_cast<int*>(next + 1);
   e = cudaMemsetAsync(acc, 0, (size_t)ng * sizeof(double) + 16, st);
   const long long total = (long long)J.p.W * J.p.H * J.p.slots;
-  const size_t shared =
-      sizeof(AdjTrav) * (kPathThreads / 32) + (nmats <= kSharedMats ? (size_t)ng * sizeof(float) : 0);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+  const size_t fixed = sizeof(AdjTrav) * (kPathThreads / 32);
+  const size_t shared = fixed + (nmats <= kSharedMats ? (size_t)ng * sizeof(float) : 0);
+  // the limit belongs to the kernel, not to the call: every call sets the same, so
+  // none lowers it between another thread's call and its launch
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(fixed + sizeof(float) * kSharedMats * kGradPerMat));
   if (e == cudaSuccess && total > 0) {
     // the slots over all warps first (kInStep lanes), then over their lanes, kTurns to
     // a lane before it takes more lanes

@@ -303,3 +303,36 @@ def test_gradient_is_the_sum_of_its_parts():
     err = np.abs(whole - parts.sum(0))
     print("largest relative difference", (err / np.maximum(np.abs(whole), 1e-30))[:, cols].max())
     assert (err <= tol)[:, cols].all(), (err / np.maximum(tol, 1e-30))[:, cols]
+
+
+def test_calls_of_scenes_with_other_material_counts_run_side_by_side():
+    """Four threads, two scenes: the size of the kernel's gradient table depends
+    on the scene's material count, and no call's launch depends on another's."""
+    import threading
+    large = scenes.cornell16()
+    large.materials = np.concatenate([large.materials] + [large.materials[:1]] * 900)
+    a = api.RenderArgs.from_camera(scenes.cornell_camera(1, 1, 2, max_depth=2), seed=1)
+    g = torch.ones(1, 3, device="cuda")
+    errors = []
+
+    def work(m, ph, st, out, want):
+        try:
+            for _ in range(3000):
+                api.adjoint(m, a, ph, g, out, stream=st)
+            np.testing.assert_allclose(out.cpu().numpy(), want, rtol=1e-6, atol=1e-7)
+        except Exception as e:  # raised in the test's own thread below
+            errors.append(e)
+
+    threads = []
+    for s in (scenes.cornell16(), large) * 2:
+        m = api.Model(s)
+        ph = api.render(m, a)
+        want = api.adjoint(m, a, ph, g).cpu().numpy()
+        threads.append(threading.Thread(target=work, args=(m, ph, torch.cuda.Stream(), torch.zeros(
+            want.shape, device="cuda"), want)))
+    torch.cuda.synchronize()
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
