@@ -714,7 +714,7 @@ rmn_status rmn_batch_create(const rmn_batch_item* items, int32_t n, const rmn_ba
   rmn_batch* bt = new (std::nothrow) rmn_batch();
   if (!bt) return fail(RMN_ERR_OUT_OF_MEMORY, "host allocation failed");
   r = batch_create(its.data(), n, opt.use_graph != 0, opt.pool_workers, opt.lanes, opt.stack_entries,
-                   opt.ray_order, static_cast<cudaStream_t>(stream), &bt->state);
+                   opt.ray_order, static_cast<cudaStream_t>(stream), &bt->state, 1.0, true);
   if (r != RMN_OK) {
     delete bt;
     return r;

@@ -182,6 +182,7 @@ void release_cached_memory() {
     std::lock_guard<std::mutex> lock(g_status_mu);
     if (g_status_free.size() == 64 * g_status_pages.size()) {  // no call in flight
       for (int* p : g_status_pages) cudaFreeHost(p);
+      cudaGetLastError();  // after a device reset they are gone already
       g_status_pages.clear();
       g_status_free.clear();
     }

@@ -1811,7 +1811,8 @@ struct BatchState {
   JobTable table;
   Job* d_jobs = nullptr;
   CtlBlock* d_ctl = nullptr;
-  int* d_status = nullptr;    // pinned status word (acquire_status)
+  int* d_status = nullptr;    // pinned status word: the call's (acquire_status), or of a held batch its own
+  bool held = false;          // the batch outlives the call that created it
   float4* d_parts = nullptr;
   int lanes = 1;
   bool alpha = false;         // some job's scene has alpha-tested materials
@@ -2194,7 +2195,8 @@ void batch_destroy(BatchState* b, bool idle) {
   // the blocks go back to the cache for the next batch: no work of this
   // batch may still run on them (cudaFree would have waited likewise)
   if (!idle) cudaDeviceSynchronize();
-  release_status(b->d_status);
+  if (!b->held) release_status(b->d_status);
+  else if (b->d_status) cudaFreeHost(b->d_status);
   if (b->h_jobs) cudaFreeHost(b->h_jobs);
   for (void* p : b->allocs) cached_free(p);
   delete b;
@@ -2260,7 +2262,8 @@ int default_stack_entries(const RenderItem* items, int n) {
 }
 
 rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int pool_workers, int lanes,
-                        int stack_entries, int ray_order, cudaStream_t st, BatchState** out, double proxy_of) {
+                        int stack_entries, int ray_order, cudaStream_t st, BatchState** out, double proxy_of,
+                        bool held) {
   *out = nullptr;
   // the traversal stack must hold every item's deepest path of deferred
   // children; a larger one only costs occupancy
@@ -2393,7 +2396,13 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
     }
   }
   if (e == cudaSuccess) e = cudaMemcpy(b->d_jobs, b->table.jobs.data(), jb, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = acquire_status(&b->d_status);
+  b->held = held;
+  if (e == cudaSuccess && held) {
+    e = cudaHostAlloc(reinterpret_cast<void**>(&b->d_status), sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e == cudaSuccess) *b->d_status = 0;
+  } else if (e == cudaSuccess) {
+    e = acquire_status(&b->d_status);
+  }
   // streams and events for the lanes beside the caller's stream, and one to
   // capture graphs on
   for (int l = use_graph ? 0 : 1; l < b->lanes && e == cudaSuccess; ++l) {

@@ -145,7 +145,9 @@ void release_cached_memory();
 cudaError_t staging_malloc(void** p, size_t bytes, cudaStream_t st);
 // A status word of one call: pinned host memory that kernels write and the host
 // reads once the call's stream is synchronised (no device word to clear, no
-// copy back). acquire gives it zeroed; the words are kept for later calls.
+// copy back). acquire gives it zeroed; the words are kept for later calls. What
+// outlives a call has a word of its own, so that release_cached_memory, called
+// after a device reset, finds none in use and forgets them all.
 cudaError_t acquire_status(int** word);
 void release_status(int* word);
 // SMs of the current device, and the blocks of `threads` threads (no dynamic
@@ -161,8 +163,10 @@ void noalloc_forget_addresses();
 // ray_order: 1 bins each ray queue by origin cell and direction octant
 // before it is traced, 0 traces the queues in the order they were filled.
 // proxy_of: the batch stands for one 1 / proxy_of times its size (autotuner).
+// held: the batch outlives the call that creates it.
 rmn_status batch_create(const RenderItem* items, int n, bool use_graph, int pool_workers, int lanes,
-                        int stack_entries, int ray_order, cudaStream_t st, BatchState** out, double proxy_of = 1.0);
+                        int stack_entries, int ray_order, cudaStream_t st, BatchState** out, double proxy_of = 1.0,
+                        bool held = false);
 // The traversal stack the library picks for these items (RMN_STACK_SMALL when
 // every tree is at most RMN_STACK_SMALL - 1 deep, else RMN_STACK).
 int default_stack_entries(const RenderItem* items, int n);

@@ -250,3 +250,54 @@ def test_ray_counts(port, n):
     assert np.array_equal(face, of) and np.array_equal(t, ot)
     rays = scenes.random_rays(n, 11, shadow=True)
     assert np.array_equal(m.rayHit_test(torch.from_numpy(rays).cuda()).cpu().numpy(), o.trace_shadow(rays))
+
+
+def test_queries_after_a_reset_with_a_batch_alive():
+    """cudaDeviceReset takes the library's pinned memory with it; after
+    rmn_release_cached_memory a query on a new scene works although a batch from
+    before the reset has not been destroyed (in a process of its own, whose
+    buffers come from the runtime itself)."""
+    code = """
+import ctypes as C, os
+import numpy as np
+from raym0nade_gb300 import _lib, api, scenes
+lib = _lib.load()
+rt = next(C.CDLL(line.split()[-1]) for line in open("/proc/self/maps") if "libcudart" in line)
+
+class Dev:  # a device buffer with the attributes that api reads of a numpy array
+    def __init__(self, nbytes, data=None):
+        p = C.c_void_p()
+        assert rt.cudaMalloc(C.byref(p), C.c_size_t(nbytes)) == 0
+        if data is not None:
+            assert rt.cudaMemcpy(p, C.c_void_p(data.ctypes.data), C.c_size_t(nbytes), 1) == 0
+        self.data = p.value
+    ctypes = property(lambda self: self)
+
+rays = scenes.random_rays(64, 1)
+old = api.Model(scenes.cornell())
+lib.rmn_trace_closest(old.handle, Dev(rays.nbytes, rays).data, 64, Dev(1024).data, None)
+cam = scenes.cornell_camera(8, 8, 1)
+ph = api.Photo(8, 8, device=False)
+for k in ("radiance_Dd", "radiance_Ds", "radiance_Id", "radiance_Is"):
+    setattr(ph, k, Dev(8 * 8 * 16))
+ph.Gbuffer, ph.dropped = Dev(8 * 8 * 4 * api.GBUFFER_FLOATS), None
+batch = api.Batch([(old, api.RenderArgs.from_camera(cam), ph)], use_graph=False)
+assert rt.cudaDeviceReset() == 0
+assert lib.rmn_release_cached_memory() == 0
+m = api.Model(scenes.cornell())
+out = Dev(1024)
+for _ in range(70):
+    assert lib.rmn_trace_closest(m.handle, Dev(rays.nbytes, rays).data, 64, out.data, None) == 0, lib.rmn_last_error()
+got = np.empty((64, 4), np.float32)
+assert rt.cudaMemcpy(C.c_void_p(got.ctypes.data), C.c_void_p(out.data), C.c_size_t(1024), 2) == 0
+print("hits", int((got.view(np.int32)[:, 0] >= 0).sum()), flush=True)
+os._exit(0)  # the objects from before the reset are not destroyed
+"""
+    import subprocess
+    import sys
+    p = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert p.returncode == 0, (p.returncode, p.stderr[-2000:])
+    rays = torch.from_numpy(scenes.random_rays(64, 1)).cuda()
+    face, _, _ = api.split_hits(api.Model(scenes.cornell()).rayHit(rays))
+    assert p.stdout.split()[-1] == str(int((face >= 0).sum()))
