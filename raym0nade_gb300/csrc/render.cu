@@ -2395,7 +2395,11 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
       alloc((void**)&bb.bins, sizeof(unsigned) * 2 * kBins);
     }
   }
-  if (e == cudaSuccess) e = cudaMemcpy(b->d_jobs, b->table.jobs.data(), jb, cudaMemcpyHostToDevice);
+  // the job table, before the first render: on this call's own stream, or, for a
+  // held batch, which may be rendered on any, before the call returns
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(b->d_jobs, b->table.jobs.data(), jb, cudaMemcpyHostToDevice, held ? nullptr : st);
+  if (e == cudaSuccess && held) e = cudaStreamSynchronize(nullptr);
   b->held = held;
   if (e == cudaSuccess && held) {
     e = cudaHostAlloc(reinterpret_cast<void**>(&b->d_status), sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
@@ -2422,7 +2426,6 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
     batch_destroy(b, false);
     return cuda_fail(e, "batch setup");
   }
-  (void)st;
   *out = b;
   return RMN_OK;
 }

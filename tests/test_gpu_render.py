@@ -342,3 +342,22 @@ def test_batch_update_moves_cameras():
     with pytest.raises(api.RmnError) as e:
         b.update(bad)
     assert e.value.status == 1
+
+
+def test_render_does_not_wait_for_another_stream():
+    """A render on a stream of its own neither waits for the work of the
+    default stream nor leaves its set-up to it: the job table is copied on the
+    render's stream."""
+    m = api.Model(scenes.cornell())
+    a = api.RenderArgs.from_camera(scenes.cornell_camera(24, 24, 4), seed=6)
+    ref = _photo_np(api.render(m, a))
+    own, ph = torch.cuda.Stream(), api.Photo(24, 24)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(1 << 30)  # half a second
+    slept = torch.cuda.Event()
+    slept.record()
+    api.render(m, a, ph, stream=own)
+    assert not slept.query()
+    torch.cuda.synchronize()
+    for x, y in zip(_photo_np(ph), ref):
+        assert np.array_equal(x, y, equal_nan=True)
