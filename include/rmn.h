@@ -295,8 +295,8 @@ rmn_status rmn_batch_destroy(rmn_batch* batch);
  * (112 B per unit of every item, at its slots_per_unit or the library's
  * default split) and the worker pool (per worker its path state, shadow-ray
  * slots and queue entries, times pool_workers per lane -- at most one
- * worker per unit -- times lanes; the library's default pool counted at its
- * full 2^22 per lane). No counterpart in the reference; for callers that
+ * worker per unit, and in a batch of few units 1024 per SM on one lane -- times
+ * lanes; the library's default pool counted at its full 2^22 per lane). No counterpart in the reference; for callers that
  * plan device memory, and the autotuner's memory cap. */
 rmn_status rmn_batch_device_bytes(const rmn_batch_item* items, int32_t n, const rmn_batch_options* options,
                                   int64_t* out);

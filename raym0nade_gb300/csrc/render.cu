@@ -2004,6 +2004,28 @@ static long long block_capacity() { return (long long)device_sms() * kLocalWorke
 // against 4.3.
 constexpr long long kDirectUnits = 400000;
 
+// How a batch is rendered: by block_kernel alone (direct) or the wavefront, and
+// with how many lanes and, before the number of units and the free memory have
+// their say, workers a lane. proxy_of: as in batch_create; a proxy of a larger
+// batch is rendered as that batch would be.
+struct Shape {
+  bool direct;
+  int lanes;
+  long long per;
+};
+static Shape batch_shape(const JobTable& t, int pool_workers, int lanes, double proxy_of) {
+  Shape s;
+  s.direct = (double)t.total_units <= proxy_of * (double)kDirectUnits;
+  s.per = pool_workers > 0 ? pool_workers : kDefaultPoolWorkers;
+  if (s.direct) {
+    s.lanes = 1;
+    s.per = std::min(s.per, block_capacity());  // no more than are resident
+  } else {
+    s.lanes = lanes > 0 ? std::min(lanes, kMaxLanes) : default_lanes((long long)((double)t.total_units / proxy_of));
+  }
+  return s;
+}
+
 // block_kernel over the n workers of one lane that wait at the end of an
 // iteration of parity 1, or were seeded.
 static cudaError_t launch_block(BatchState* b, int lane, long long n, cudaStream_t st) {
@@ -2284,19 +2306,14 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
   b->table.slots = S_def;
   b->use_graph = use_graph;
   b->binned = ray_order != 0;
-  b->lanes = lanes > 0 ? std::min(lanes, kMaxLanes)
-                       : default_lanes((long long)((double)b->table.total_units / proxy_of));
-  // workers per lane; no more lanes and workers than there are units, nor, for a
-  // render without wavefront, than are resident; the default pool halves while
-  // the workers would take more than a quarter of the free device memory
-  long long per = pool_workers > 0 ? pool_workers : kDefaultPoolWorkers;
-  // a proxy of a larger batch is rendered as that batch would be
-  b->direct = (double)b->table.total_units <= proxy_of * (double)kDirectUnits;
+  const Shape shape = batch_shape(b->table, pool_workers, lanes, proxy_of);
+  b->direct = shape.direct;
+  b->lanes = shape.lanes;
   b->tail = (long long)(proxy_of * (double)block_capacity());
-  if (b->direct) {
-    b->lanes = 1;
-    per = std::min(per, std::min(block_capacity(), b->table.total_units));
-  }
+  // workers per lane; no more lanes and workers than there are units; the
+  // default pool halves while the workers would take more than a quarter of the
+  // free device memory
+  long long per = shape.per;
   if (pool_workers <= 0) {
     bool glass = false, tex = false;
     for (const Job& j : b->table.jobs) {
@@ -2490,9 +2507,9 @@ size_t batch_device_bytes(const RenderItem* items_in, int n, int pool_workers, i
     glass = glass || j.p.glass;
     tex = tex || j.s.has_tex;
   }
-  const int nl = lanes > 0 ? std::min(lanes, kMaxLanes) : default_lanes(t.total_units);
-  long long per = pool_workers > 0 ? pool_workers : kDefaultPoolWorkers;
-  per = std::min<long long>(per, (t.total_units + nl - 1) / nl);
+  const Shape shape = batch_shape(t, pool_workers, lanes, 1.0);
+  const int nl = shape.lanes;
+  const long long per = std::min<long long>(shape.per, (t.total_units + nl - 1) / nl);
   // binning: the reordered queues and each entry's bucket, per worker; the
   // bucket counters per lane
   const size_t bin_bytes =

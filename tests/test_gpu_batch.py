@@ -153,3 +153,21 @@ def test_default_split_depends_on_the_render_alone():
     torch.cuda.synchronize()
     for x, y in zip(_photo_np(ph), ref):
         assert np.array_equal(x, y, equal_nan=True)
+
+
+@pytest.mark.parametrize("lanes", [0, 1, 3])
+def test_device_bytes_of_a_batch_of_few_units(lanes):
+    """256 x 256 at 16 spp, 5 units a pixel: rendered on one lane with at most
+    1024 workers per SM, whatever the pool and the lanes asked for, and
+    rmn_batch_device_bytes counts those."""
+    m = api.Model(scenes.cornell())
+    a = api.RenderArgs.from_camera(scenes.cornell_camera(256, 256, 16), seed=1)
+    items = [(m, a, api.Photo(256, 256))]
+    units = 256 * 256 * 5
+    held = 1024 * torch.cuda.get_device_properties(0).multi_processor_count
+    one, two = (api.batch_device_bytes(items, n, 1) for n in (128, 256))
+    per_worker = (two - one) / 128
+    assert held < units
+    assert api.batch_device_bytes(items, 0, lanes) == units * 112 + held * per_worker
+    assert api.batch_device_bytes(items, 1 << 20, lanes) == units * 112 + held * per_worker
+    assert api.batch_device_bytes(items, 1000, lanes) == units * 112 + 1000 * per_worker
