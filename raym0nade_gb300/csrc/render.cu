@@ -1805,6 +1805,8 @@ struct JobTable {
   std::vector<int> slots; // slots per unit chosen for an item that left it to the library (else 0)
   int total_pix = 0;
   long long total_units = 0;
+  long long work = 0;     // the units there would be at 2 slots each, the default split of small items
+  bool glass = false;     // some item's scene has transmissive or half-opaque materials
 };
 
 struct BatchState {
@@ -1861,7 +1863,8 @@ static void build_jobs(const RenderItem* items, int n, JobTable* t) {
   t->jobs.clear();
   t->item = order;
   t->total_pix = 0;
-  t->total_units = 0;
+  t->total_units = t->work = 0;
+  t->glass = false;
   for (int i : order) {
     const RenderItem& it = items[i];
     Job j;
@@ -1877,6 +1880,10 @@ static void build_jobs(const RenderItem* items, int n, JobTable* t) {
     j.unit_begin = t->total_units;
     t->total_pix += j.p.W * j.p.H;
     t->total_units += (long long)j.p.W * j.p.H * j.p.K;
+    const int path_slots = (j.p.glass ? j.p.slots16 : j.p.slots) - j.p.spp_d;
+    const int split = (j.p.spp_d + kLightSlotsPerUnit - 1) / kLightSlotsPerUnit + (path_slots + 1) / 2;
+    t->work += (long long)j.p.W * j.p.H * std::max(1, split);
+    t->glass = t->glass || j.p.glass;
     t->jobs.push_back(j);
   }
 }
@@ -2001,8 +2008,17 @@ static long long block_capacity() { return (long long)device_sms() * kLocalWorke
 // kernels: Cornell 256x256, 16 spp, 328 k units: 1.74 ms against 2.0 with the
 // wavefront first; the textured room 320x240, 8 spp, 230 k: 1.5 against 1.84; a
 // terrain 480x270, 16 spp, 648 k: 2.9 against 2.75; Cornell 64 spp, 1.05 M: 5.2
-// against 4.3.
-constexpr long long kDirectUnits = 400000;
+// against 4.3. On 152 SMs the line is at 400 k units.
+constexpr long long kDirectUnits = 2632;  // per SM
+// Units may hold any number of slots, so a second line counts them at 2 slots
+// each, on 152 SMs at 608 k. One unit a pixel, block_kernel alone against the
+// wavefront first: 300x300, 16 spp, 450 k: Cornell 2.31 and 2.45 ms, terrain 2.06 and
+// 1.92; 32 spp, 720 k: Cornell 4.16 and 4.14, terrain 3.84 and 3.29, textured room
+// 5.1 and 4.9; 600x600, 1024 spp, 59 M: 400 and 365, 330 and 238, 364 and 321. With
+// glass the first line alone counts: a pixel behind it has up to 16 times the
+// slots of another, and the wavefront waits for the last units (300x300, 16 spp,
+// 4.3 M: 41 and 54 ms; 600x600, 64 spp, 226 and 243).
+constexpr long long kDirectWork = 4000;  // per SM
 
 // How a batch is rendered: by block_kernel alone (direct) or the wavefront, and
 // with how many lanes and, before the number of units and the free memory have
@@ -2015,7 +2031,8 @@ struct Shape {
 };
 static Shape batch_shape(const JobTable& t, int pool_workers, int lanes, double proxy_of) {
   Shape s;
-  s.direct = (double)t.total_units <= proxy_of * (double)kDirectUnits;
+  const double sms = proxy_of * (double)device_sms();
+  s.direct = (double)t.total_units <= sms * kDirectUnits && (t.glass || (double)t.work <= sms * kDirectWork);
   s.per = pool_workers > 0 ? pool_workers : kDefaultPoolWorkers;
   if (s.direct) {
     s.lanes = 1;

@@ -171,3 +171,20 @@ def test_device_bytes_of_a_batch_of_few_units(lanes):
     assert api.batch_device_bytes(items, 0, lanes) == units * 112 + held * per_worker
     assert api.batch_device_bytes(items, 1 << 20, lanes) == units * 112 + held * per_worker
     assert api.batch_device_bytes(items, 1000, lanes) == units * 112 + 1000 * per_worker
+
+
+@pytest.mark.parametrize("spp,direct", [(1, True), (4, True), (8, False), (64, False), (4096, False)])
+def test_few_units_of_many_slots_are_much_work(spp, direct):
+    """A render of one unit a pixel and 2000 units per SM: it goes without the
+    wavefront, on 1024 workers per SM, only while its sample slots would make no
+    more than 4000 units of two (the light samples: of eight) per SM; with
+    glass, whatever their number."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    w = int((2000 * sms) ** 0.5)
+    spp_d = int(np.float32(spp) * np.float32(0.7))
+    assert direct == (w * w * ((spp_d + 7) // 8 + (spp - spp_d + 1) // 2) <= 4000 * sms)
+    for scene, held in ((scenes.cornell(), 1024 * sms if direct else w * w), (scenes.cornell_glass(), 1024 * sms)):
+        a = api.RenderArgs.from_camera(scenes.cornell_camera(w, w, spp), lanes_per_pixel=1)
+        items = [(api.Model(scene), a, api.Photo(8, 8))]
+        full, one, two = (api.batch_device_bytes(items, n, 1) for n in (1 << 20, 128, 256))
+        assert full == one + (held - 128) * (two - one) // 128
