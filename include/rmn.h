@@ -314,7 +314,9 @@ rmn_status rmn_batch_device_bytes(const rmn_batch_item* items, int32_t n, const 
  * of those
  * once more with the other traversal stack build where the batch's trees
  * allow both (27 entries instead of 23), then the fastest with its ray
- * queues binned (ray_order 1). Returns the fastest. Set each item's
+ * queues binned (ray_order 1). Where a candidate's batch is rendered without
+ * the wavefront (rmn_batch_options), its pools, lanes and ray order are not
+ * told apart: one of them is timed. Returns the fastest. Set each item's
  * slots_per_unit and the batch's pool_workers, lanes, stack_entries and
  * ray_order from the result. The images do not depend on the choice
  * beyond float summation order across units (slots_per_unit); pool size,

@@ -785,6 +785,16 @@ rmn_status rmn_batch_autotune(const rmn_batch_item* items, int32_t n, float pixe
     for (RenderItem& it : f) it.args.slots_per_unit = slots;
     return batch_device_bytes(f.data(), n, pool, lanes, order) <= free_b / 2;
   };
+  // candidates that differ only in what a batch of little work does without
+  // are one
+  auto direct = [&](int slots) {
+    std::vector<RenderItem> f = full;
+    for (RenderItem& it : f) {
+      it.args.lanes_per_pixel = 0;
+      if (slots) it.args.slots_per_unit = slots;
+    }
+    return batch_is_direct(f.data(), n);
+  };
   // the batch cannot be built at all when its default unit records and the
   // smallest pool exceed what is free
   if (batch_device_bytes(full.data(), n, 4096, 1) > free_b)
@@ -855,8 +865,8 @@ rmn_status rmn_batch_autotune(const rmn_batch_item* items, int32_t n, float pixe
       cl = best.lanes;
       ck = stack_pass ? RMN_STACK : best.stack_entries;
       co = order_pass ? 1 : 0;
-      if (order_pass && !fits(cs, cp, cl, co)) continue;
-    } else if (!is_default && !fits(cs, cp, cl, 0)) {
+      if (order_pass && (!fits(cs, cp, cl, co) || direct(cs))) continue;
+    } else if (!is_default && (!fits(cs, cp, cl, 0) || ((pi > 0 || li > 0) && direct(cs)))) {
       continue;
     }
     for (size_t i = 0; i < its.size(); ++i) its[i].args.slots_per_unit = cs == 0 ? proxy_slots[i] : cs;

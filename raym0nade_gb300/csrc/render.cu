@@ -2507,11 +2507,8 @@ rmn_status batch_update(BatchState* b, const rmn_render_args* args, int n, cudaS
 
 size_t batch_job_bytes() { return sizeof(Job); }
 
-// Device bytes batch_create would take for these items: the unit partials,
-// and per worker its state, shadow-ray slots and queue entries (media and
-// ray differentials where a scene needs them).
-size_t batch_device_bytes(const RenderItem* items_in, int n, int pool_workers, int lanes, int ray_order) {
-  // items that leave the unit split open take the library's default
+// The job table of items of which some leave the unit split to the library.
+static JobTable split_jobs(const RenderItem* items_in, int n) {
   std::vector<RenderItem> items(items_in, items_in + n);
   std::vector<int> S(n, 0);
   default_slots_per_unit(items_in, n, S.data());
@@ -2519,6 +2516,14 @@ size_t batch_device_bytes(const RenderItem* items_in, int n, int pool_workers, i
     if (S[i]) items[i].args.slots_per_unit = S[i];
   JobTable t;
   build_jobs(items.data(), n, &t);
+  return t;
+}
+
+// Device bytes batch_create would take for these items: the unit partials,
+// and per worker its state, shadow-ray slots and queue entries (media and
+// ray differentials where a scene needs them).
+size_t batch_device_bytes(const RenderItem* items_in, int n, int pool_workers, int lanes, int ray_order) {
+  const JobTable t = split_jobs(items_in, n);
   bool glass = false, tex = false;
   for (const Job& j : t.jobs) {
     glass = glass || j.p.glass;
@@ -2536,6 +2541,9 @@ size_t batch_device_bytes(const RenderItem* items_in, int n, int pool_workers, i
   return sizeof(float4) * RMN_PART_F4 * (size_t)t.total_units + worker_bytes(glass, tex) * (size_t)per * nl +
          bin_bytes;
 }
+
+bool batch_is_direct(const RenderItem* items, int n) { return batch_shape(split_jobs(items, n), 0, 0, 1.0).direct; }
+
 int batch_items(const BatchState* b) { return (int)b->table.jobs.size(); }
 
 rmn_status batch_status(BatchState* b, cudaStream_t st) {

@@ -178,6 +178,9 @@ rmn_status batch_update(BatchState* b, const rmn_render_args* args, int n, cudaS
 size_t batch_job_bytes();
 size_t batch_device_bytes(const RenderItem* items, int n, int pool_workers, int lanes, int ray_order = 0);
 void default_slots_per_unit(const RenderItem* items, int n, int* S);
+// Whether these items make a batch that is rendered without the wavefront:
+// its lanes, ray order and any pool above 1024 workers per SM then have no part.
+bool batch_is_direct(const RenderItem* items, int n);
 int batch_items(const BatchState* b);
 rmn_status batch_status(BatchState* b, cudaStream_t st);
 rmn_status batch_profile(BatchState* b, cudaStream_t st, RenderProfileData* prof);

@@ -188,3 +188,10 @@ def test_few_units_of_many_slots_are_much_work(spp, direct):
         items = [(api.Model(scene), a, api.Photo(8, 8))]
         full, one, two = (api.batch_device_bytes(items, n, 1) for n in (1 << 20, 128, 256))
         assert full == one + (held - 128) * (two - one) // 128
+
+
+def test_autotune_times_what_differs():
+    """A batch rendered without the wavefront differs by its slots per unit and
+    its stack alone: the library's choice, four splits and the deeper stack."""
+    res = api.autotune(_uneven_items(), pixel_fraction=0.25)
+    assert res["candidates"] == 6 and res["ray_order"] == 0
