@@ -2453,8 +2453,10 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
     // join through events between the lane streams), so their kernels overlap.
     cudaStream_t c0 = b->ls[0];
     e = capture(c0, [&] { return b->direct ? launch_direct(b, c0) : launch_init(b, c0, nullptr); }, &b->init_exec);
-    if (e == cudaSuccess) e = capture(c0, [&] { return launch_lanes(b, c0, nullptr, nullptr); }, &b->chunk_exec);
-    if (e == cudaSuccess) e = capture(c0, [&] { return launch_finalize(b, c0); }, &b->fin_exec);
+    // a direct batch's first graph is the whole render
+    if (e == cudaSuccess && !b->direct)
+      e = capture(c0, [&] { return launch_lanes(b, c0, nullptr, nullptr); }, &b->chunk_exec);
+    if (e == cudaSuccess && !b->direct) e = capture(c0, [&] { return launch_finalize(b, c0); }, &b->fin_exec);
   }
   if (e != cudaSuccess) {
     batch_destroy(b, false);
