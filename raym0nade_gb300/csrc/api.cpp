@@ -72,9 +72,11 @@ void release(Arg& a, cudaStream_t st) {
 
 // Status word of one call: kernels on the call's stream write it.
 struct Status {
+  rmn::StatusWord status;
   int* word = nullptr;
   rmn_status init() {
-    cudaError_t e = rmn::acquire_status(&word);
+    cudaError_t e = rmn::acquire_status(&status);
+    word = status.word;
     if (e != cudaSuccess) return cuda_fail(e, "pinned allocation (status)");
     return RMN_OK;
   }
@@ -86,7 +88,7 @@ struct Status {
     return RMN_OK;
   }
   void free() {
-    rmn::release_status(word);
+    rmn::release_status(&status);
     word = nullptr;
   }
 };

@@ -8,7 +8,7 @@
 // to kCacheLimit bytes per device; rmn_release_cached_memory frees them.
 //
 // The calls' short-lived buffers (host arrays staged through the device,
-// intermediate images, status words) are stream-ordered allocations from a
+// intermediate images) are stream-ordered allocations from a
 // memory pool of the library's own per device, which keeps up to
 // kStagingKeep bytes across stream synchronisations. The device's default
 // pool gives its memory back at every synchronisation (release threshold
@@ -60,12 +60,14 @@ cudaError_t staging_pool(cudaMemPool_t* out) {
   return cudaSuccess;
 }
 
-// Status words, 64 bytes apart in pinned pages of 64: at most as many as calls
-// were ever in flight at once, rounded up to a page.
-constexpr int kStatusStride = 16;
+// Status words, 64 bytes apart in pinned pages of 64: at most as many as were
+// ever in use at once, rounded up to a page. A page whose words are in use when
+// the cached memory is given back goes with its last word; no word of it is
+// handed out again, since a device reset may have unmapped it.
+constexpr int kStatusStride = 16, kStatusWords = 64;
 std::mutex g_status_mu;
-std::vector<int*> g_status_free;
-std::vector<int*> g_status_pages;
+std::vector<StatusWord> g_status_free;
+std::vector<StatusPage*> g_status_pages;
 
 // Launch limits by device and kernel: they do not change.
 std::mutex g_limit_mu;
@@ -86,6 +88,20 @@ void release_all(DeviceCache& c) {
   c.cached = 0;
 }
 
+}  // namespace
+
+struct StatusPage {
+  int* words = nullptr;
+  int used = 0;      // words in use
+  bool old = false;  // given back while some were
+};
+
+namespace {
+void free_page(StatusPage* p) {
+  cudaFreeHost(p->words);
+  cudaGetLastError();  // after a device reset it is gone already
+  delete p;
+}
 }  // namespace
 
 cudaError_t cached_malloc(void** p, size_t bytes) {
@@ -138,26 +154,32 @@ cudaError_t staging_malloc(void** p, size_t bytes, cudaStream_t st) {
   return cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, st);
 }
 
-cudaError_t acquire_status(int** word) {
+cudaError_t acquire_status(StatusWord* w) {
   std::lock_guard<std::mutex> lock(g_status_mu);
   if (g_status_free.empty()) {
-    int* page = nullptr;
-    cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&page), 64 * kStatusStride * sizeof(int),
+    int* words = nullptr;
+    cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&words), kStatusWords * kStatusStride * sizeof(int),
                                   cudaHostAllocPortable | cudaHostAllocMapped);
     if (e != cudaSuccess) return e;
-    g_status_pages.push_back(page);
-    for (int i = 0; i < 64; ++i) g_status_free.push_back(page + i * kStatusStride);
+    StatusPage* p = new StatusPage();
+    p->words = words;
+    g_status_pages.push_back(p);
+    for (int i = 0; i < kStatusWords; ++i) g_status_free.push_back({words + i * kStatusStride, p});
   }
-  *word = g_status_free.back();
+  *w = g_status_free.back();
   g_status_free.pop_back();
-  **word = 0;
+  w->page->used++;
+  *w->word = 0;
   return cudaSuccess;
 }
 
-void release_status(int* word) {
-  if (!word) return;
+void release_status(StatusWord* w) {
+  if (!w->word) return;
   std::lock_guard<std::mutex> lock(g_status_mu);
-  g_status_free.push_back(word);
+  w->page->used--;
+  if (!w->page->old) g_status_free.push_back(*w);
+  else if (w->page->used == 0) free_page(w->page);
+  *w = StatusWord{};
 }
 
 int device_sms() {
@@ -180,12 +202,12 @@ int blocks_per_sm(const void* kernel, int threads) {
 void release_cached_memory() {
   {
     std::lock_guard<std::mutex> lock(g_status_mu);
-    if (g_status_free.size() == 64 * g_status_pages.size()) {  // no call in flight
-      for (int* p : g_status_pages) cudaFreeHost(p);
-      cudaGetLastError();  // after a device reset they are gone already
-      g_status_pages.clear();
-      g_status_free.clear();
+    for (StatusPage* p : g_status_pages) {
+      if (p->used == 0) free_page(p);
+      else p->old = true;
     }
+    g_status_pages.clear();
+    g_status_free.clear();
   }
   {
     std::lock_guard<std::mutex> lock(g_pool_mu);

@@ -1813,8 +1813,8 @@ struct BatchState {
   JobTable table;
   Job* d_jobs = nullptr;
   CtlBlock* d_ctl = nullptr;
-  int* d_status = nullptr;    // pinned status word: the call's (acquire_status), or of a held batch its own
-  bool held = false;          // the batch outlives the call that created it
+  int* d_status = nullptr;    // pinned status word
+  StatusWord status;
   float4* d_parts = nullptr;
   int lanes = 1;
   bool alpha = false;         // some job's scene has alpha-tested materials
@@ -2234,8 +2234,7 @@ void batch_destroy(BatchState* b, bool idle) {
   // the blocks go back to the cache for the next batch: no work of this
   // batch may still run on them (cudaFree would have waited likewise)
   if (!idle) cudaDeviceSynchronize();
-  if (!b->held) release_status(b->d_status);
-  else if (b->d_status) cudaFreeHost(b->d_status);
+  release_status(&b->status);
   if (b->h_jobs) cudaFreeHost(b->h_jobs);
   for (void* p : b->allocs) cached_free(p);
   delete b;
@@ -2434,13 +2433,8 @@ rmn_status batch_create(const RenderItem* items_in, int n, bool use_graph, int p
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(b->d_jobs, b->table.jobs.data(), jb, cudaMemcpyHostToDevice, held ? nullptr : st);
   if (e == cudaSuccess && held) e = cudaStreamSynchronize(nullptr);
-  b->held = held;
-  if (e == cudaSuccess && held) {
-    e = cudaHostAlloc(reinterpret_cast<void**>(&b->d_status), sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
-    if (e == cudaSuccess) *b->d_status = 0;
-  } else if (e == cudaSuccess) {
-    e = acquire_status(&b->d_status);
-  }
+  if (e == cudaSuccess) e = acquire_status(&b->status);
+  b->d_status = b->status.word;
   // streams and events for the lanes beside the caller's stream, and one to
   // capture graphs on
   for (int l = use_graph ? 0 : 1; l < b->lanes && e == cudaSuccess; ++l) {

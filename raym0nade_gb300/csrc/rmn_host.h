@@ -143,13 +143,16 @@ void release_cached_memory();
 // A stream-ordered allocation from the library's staging pool (devmem.cpp),
 // freed with cudaFreeAsync.
 cudaError_t staging_malloc(void** p, size_t bytes, cudaStream_t st);
-// A status word of one call: pinned host memory that kernels write and the host
-// reads once the call's stream is synchronised (no device word to clear, no
-// copy back). acquire gives it zeroed; the words are kept for later calls. What
-// outlives a call has a word of its own, so that release_cached_memory, called
-// after a device reset, finds none in use and forgets them all.
-cudaError_t acquire_status(int** word);
-void release_status(int* word);
+// A status word of a call or a batch: pinned host memory that kernels write and
+// the host reads once the stream is synchronised (no device word to clear, no
+// copy back). acquire gives it zeroed; the words are kept for later use.
+struct StatusPage;
+struct StatusWord {
+  int* word = nullptr;
+  StatusPage* page = nullptr;
+};
+cudaError_t acquire_status(StatusWord* w);
+void release_status(StatusWord* w);
 // SMs of the current device, and the blocks of `threads` threads (no dynamic
 // shared memory) an SM of it holds of a kernel: asked of the runtime once.
 int device_sms();
