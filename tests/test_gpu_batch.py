@@ -195,3 +195,47 @@ def test_autotune_times_what_differs():
     its stack alone: the library's choice, four splits and the deeper stack."""
     res = api.autotune(_uneven_items(), pixel_fraction=0.25)
     assert res["candidates"] == 6 and res["ray_order"] == 0
+
+
+def _large_items(kind):
+    """Renders of some 425,000 units in all, above the line under which a
+    batch is rendered without the wavefront; `alpha`: one with cut-outs, whose
+    shadow rays are searched in order, and one with glass."""
+    hf = scenes.heightfield(120, seed=2, extent=12.0, patch=8)
+    hf.env = scenes.sky_env(64, 32, sun_radiance=100.0, sun_diameter_deg=8.0)
+    skycam = scenes.Camera((0.3, 2.0, -0.8), (0.35, -0.45, 0.82), (0.0, -1.0, 0.0), (-1.0, 0.0, 0.0), 0.01, 192, 128, 12)
+    specs = [(scenes.cornell(), scenes.cornell_camera(224, 224, 16), 1), (hf, skycam, 2)]
+    if kind == "alpha":
+        specs += [(scenes.textured_room(), scenes.textured_camera(160, 96, 12), 3),
+                  (scenes.cornell_glass(), scenes.cornell_camera(64, 48, 4), 4)]
+    else:
+        specs += [(scenes.random_soup(20000, 5), scenes.soup_camera(160, 128, 16, 8), 5)]
+    return [(api.Model(s), api.RenderArgs.from_camera(c, seed=k), api.Photo(c.width, c.height)) for s, c, k in specs]
+
+
+@pytest.mark.parametrize("lanes", [1, 2, 3])
+@pytest.mark.parametrize("use_graph", [True, False])
+@pytest.mark.parametrize("kind", ["plain", "alpha"])
+def test_wavefront_batches_give_identical_images(kind, use_graph, lanes):
+    """The wavefront with one lane (its launches overlapped, also inside a
+    captured graph) and with several, both traversal stack builds, with and
+    without binned ray queues, its end in block_kernel, and new arguments for a
+    built batch: every item's images are those of the wavefront alone, which
+    rmn_render_profile_get renders with."""
+    import dataclasses
+    items = _large_items(kind)
+    units = (api.batch_device_bytes(items, 128, 1) - 128 * 1300) // 112
+    assert units > 2632 * torch.cuda.get_device_properties(0).multi_processor_count
+    moved = [dataclasses.replace(a, seed=a.seed + 20) for _, a, _ in items]
+    want = [[_photo_np(api.render_profile(m, b)[0]) for (m, _, _), b in zip(items, args)]
+            for args in ([a for _, a, _ in items], moved)]
+    for stack in (23, 27):
+        for order in (0, 1):
+            b = api.Batch(items, use_graph=use_graph, stack_entries=stack, ray_order=order, lanes=lanes)
+            for k in (0, 0, 1):
+                b.update([a for _, a, _ in items] if k == 0 else moved)
+                b.render()
+                torch.cuda.synchronize()
+                for (_, _, ph), ref in zip(items, want[k]):
+                    for x, y in zip(_photo_np(ph), ref):
+                        assert np.array_equal(x.view(np.int32), y.view(np.int32)), (stack, order, k)
