@@ -223,12 +223,12 @@ cudaError_t export_images(float* const* b, const float* gb, const rmn_post_args&
                           cudaStream_t st) {
   const int W = a.width, H = a.height;
   const size_t npx = (size_t)W * H;
-  const bool dof = n > RMN_EXPORTS;
-  // the linear full image; the linear base colour and the two blurred images
-  float* scratch = nullptr;
-  cudaError_t e = staging_malloc(reinterpret_cast<void**>(&scratch), npx * 12 * (dof ? 4 : 1), st);
+  // the linear full image; the base colour and the two blurred images wait in
+  // the places of the first depth-of-field exports until these are made
+  float* full = nullptr;
+  cudaError_t e = staging_malloc(reinterpret_cast<void**>(&full), npx * 12, st);
   if (e != cudaSuccess) return e;
-  float *full = scratch, *base = scratch + 3 * npx, *base_dof = scratch + 6 * npx, *full_dof = scratch + 9 * npx;
+  float *base_dof = rgb + 3 * npx * RMN_EXPORTS, *base = base_dof + 3 * npx, *full_dof = base + 3 * npx;
   DofPlan* plan = nullptr;
   auto compose = [&](int options, float* out, float* linear) {
     return launch_compose(b[0], b[1], b[2], b[3], gb, W, H, a.exposure, options, out, st, linear);
@@ -258,7 +258,7 @@ cudaError_t export_images(float* const* b, const float* gb, const rmn_post_args&
     }
   }
   dof_plan_destroy(plan, st);
-  const cudaError_t f = cudaFreeAsync(scratch, st);
+  const cudaError_t f = cudaFreeAsync(full, st);
   return e != cudaSuccess ? e : f;
 }
 

@@ -149,3 +149,27 @@ def test_render_multithread_writes_the_export_set(tmp_path):
         tag = lib.rmn_export_tag(k).decode()
         img = _read_png(str(tmp_path / "out" / f"img({tag}).png"))
         assert img.shape == (24, 32, 3)
+
+
+def test_export_set_scratch():
+    """The export set needs no more device memory than one export with depth of
+    field and FXAA and bloom's two images beside it (each call's peak is what
+    the library's pool holds after it; 32 MiB for the pool's block size)."""
+    w, h = 1920, 1080
+    rec = photo_records(96, 64, 21)
+    ph = photo_from_records(np.tile(rec, (h // 64 + 1, w // 96, 1))[:h], dict(PHOTO_POST, coc=6.0))
+    lib = api._lib.load()
+    out = torch.empty((api.EXPORTS + api.EXPORTS_DOF, h, w, 3), device="cuda")
+    one = torch.empty((h, w, 3), device="cuda")
+
+    def peak(call):
+        torch.cuda.synchronize()
+        lib.rmn_release_cached_memory()
+        free = torch.cuda.mem_get_info()[0]
+        call()
+        torch.cuda.synchronize()
+        return free - torch.cuda.mem_get_info()[0]
+
+    single = peak(lambda: ph.post_process(api.Full | api.DoDepthFieldBlur | api.DoBloom | api.DoFXAA, one))
+    whole = peak(lambda: ph.export_set(out))
+    assert 0 < single and whole <= single + 24 * w * h + (32 << 20), (single, whole)
