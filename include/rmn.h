@@ -261,13 +261,18 @@ typedef struct rmn_batch_item {
   rmn_render_args args;
   rmn_image image;
 } rmn_batch_item;
-/* Launch knobs of a batch; NULL options = {1, 0, 0}. */
+/* Launch knobs of a batch; NULL options = {1, 0, 0}. A batch of little work --
+ * at most 2632 units per SM (400,000 on 152 SMs) and, without glass, at most 4000
+ * per SM counted at two slots each -- is rendered by one kernel without the
+ * wavefront: lanes and ray_order have no part in it, and it has at most 1024
+ * workers per SM. rmn_batch_profile renders and times the wavefront all the
+ * same, rmn_render_profile_get likewise. No image depends on any of these. */
 typedef struct rmn_batch_options {
   int32_t use_graph;     /* replay the wavefront iterations from captured CUDA graphs */
   int32_t pool_workers;  /* paths in flight per lane (0: library default, 2^22, halved while the workers
                             would take over a quarter of the free device memory) */
   int32_t lanes;         /* independent wavefronts run side by side, 1..4 (0: library default, one per 2^21 work
-                            units, 1 to 3). A batch of few units is rendered without them */
+                            units, 1 to 3) */
   int32_t stack_entries; /* traversal stack, 23 or 27 entries (0: library default, the smallest that holds
                             every item's tree: 23 when all trees are at most 22 levels deep); a stack too
                             small for a tree is RMN_ERR_INVALID_ARGUMENT */

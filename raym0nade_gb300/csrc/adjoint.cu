@@ -8,8 +8,8 @@
 // Input: the G-buffer and the per-pixel dropped-sample record of a forward
 // rmn_render with the same scene and arguments, and dL/dI (3 floats per
 // pixel). Every sample slot draws from the counter-based stream keyed
-// (seed, pixel, slot), so one thread per slot replays exactly the forward's
-// path -- same hits, same branches -- without anything stored per path.
+// (seed, pixel, slot), so a lane replays exactly the forward's path of its slot
+// -- same hits, same branches -- without anything stored per path.
 //
 // Per sample s of a path (a light sample at the terminating vertex, or the
 // emitter or sky the path hits) the contribution S_s = dL/dI . dI_s is

@@ -194,7 +194,7 @@ cudaError_t launch_fxaa(const float* in, float* out, int w, int h, cudaStream_t 
     grid = dim3((w + tx - 1) / tx, (h + ty - 1) / ty);
     if ((long long)grid.x * grid.y >= 4LL * device_sms()) break;
   }
-  const int sw = tx + HALO_LO + hx, sh = ty + HALO_LO + hy;  // at most 161 x 25 or 73 x 113 floats
+  const int sw = tx + HALO_LO + hx, sh = ty + HALO_LO + hy;  // at most 161 x 26 or 74 x 113 floats
   fxaa_kernel<<<grid, dim3(BX, BY), sizeof(float) * sw * sh, stream>>>(in, out, w, h, sw, sh, tx, ty);
   return cudaGetLastError();
 }

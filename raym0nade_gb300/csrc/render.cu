@@ -67,8 +67,8 @@ struct Counters {
   unsigned long long closest, shadow, inner, leaves, tris, slots;
 };
 
-// Queue lengths of one iteration parity; cleared when an iteration of that
-// parity starts.
+// Queue lengths of one iteration parity; cleared when a render starts and, by
+// path_kernel of the iteration before, when the queues have been read.
 struct QLen {
   unsigned int c, sn;           // ray queues: closest, shadow
   unsigned int sd, nw;          // workers waiting for first-vertex / NEE shadow answers
@@ -1289,7 +1289,7 @@ __global__ void __launch_bounds__(128, RMN_OCC_BLOCKS) qocc_kernel(const Job* __
 //
 // It takes the renders, and the ends of renders, that leave the wavefront
 // empty: an iteration of the wavefront costs 100-160 us however few workers
-// are left (nine launches in a row, each a chain of dependent loads 5-20 us
+// are left (eight launches in a row, each a chain of dependent loads 5-20 us
 // long).
 //
 // The kinds of work of a stage run one after the other, all warps on the same

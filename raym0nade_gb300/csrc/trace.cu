@@ -156,9 +156,9 @@ cudaError_t launch_kernel(const DevScene& s, const float4* rays, int64_t n, floa
   int blocks = rmn::device_sms() * rmn::blocks_per_sm(kernel, threads);
   // the rays go over all the warps the device holds, `use` of a warp's lanes
   // taking one each: a warp's time is its rays' divergent steps one after the
-  // other. With 32 rays a warp while most of the device is idle, 1000 rays of the
-  // 130 k-triangle terrain take 114 us a call against 90 with one, 100 of the
-  // 1 M soup 327 against 192; from 32 rays a warp on (155,648 in all) nothing
+  // other. A whole call with 32 rays a warp, and so: 1000 rays of the 130
+  // k-triangle terrain 57 and 47 us; 100, 1000 and 20,000 of the 1 M soup 211 and
+  // 114, 331 and 214, 361 and 297; from 32 rays a warp on (155,648 in all) nothing
   // changes.
   const int64_t warps = (int64_t)blocks * (threads / 32);
   const int use = (int)std::min<int64_t>(32, (n + warps - 1) / warps);
