@@ -86,7 +86,9 @@ RMN_D float2 slab2(float a, float b, unsigned long long o, unsigned long long i)
 // rule (r.par == 0), on a box's six slab distances (lo and hi of x and y, then
 // z). The smaller of an axis's two is its entry (box_hit's choice by the sign
 // of 1/d: multiplication and subtraction round monotonely and lo <= hi).
-// Whether the box is hit is box_hit's answer; tL is box_hit's when it is.
+// Whether the box is hit is box_hit's answer; tL is box_hit's when it is. (A box
+// with NaN vertices alone under it has lo > hi: it is entered here and holds no
+// hit.)
 RMN_D bool box_run(float2 lo, float2 hi, float2 z, float tmin, float tmax, float& tL) {
   const float L1 = fmaxf(tmin, fminf(lo.x, hi.x)), R1 = fminf(tmax, fmaxf(lo.x, hi.x)) + RMN_EPS;
   const float L2 = fmaxf(L1, fminf(lo.y, hi.y)), R2 = fminf(R1, fmaxf(lo.y, hi.y)) + RMN_EPS;
